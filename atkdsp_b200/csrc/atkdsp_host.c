@@ -829,6 +829,15 @@ static int run_step_up(atkdsp_pfb *p, unsigned nel, const void *const *ins, size
         job_conv(&J[e], &C[e], cv);
     }
     T[nel] = (int)nel * tiles;
+    /* one job of few points: one CTA per hop, the job in the launch's parameters */
+    if (nel == 1 && !up_extra && !J[0].w2 && m * p->nchan <= ATKB_HOPS1_POINTS && atkb_pfb_hops_ok(&p->bank)) {
+        rc = atkb_pfb_hops1(&J[0], &C[0], (int)m, (int)p->nchan, p->d_counters, stream);
+        if (rc != ATKB_OK) return rc;
+        p->cur = (int)nxt;
+        p->lc = (unsigned)(p->lc + n - m * p->hop);
+        p->b += (int64_t)m;
+        return ATKB_OK;
+    }
     void *tb = p->d_tables;
     const int from_params = nel == 1 && !up_extra;
     if (from_params) {
@@ -867,7 +876,8 @@ static int run_step_up(atkdsp_pfb *p, unsigned nel, const void *const *ins, size
          * tile_start[njobs]); the same launch copies the nel carries */
         const int work = (int)nel * tiles + (int)nel;
         if (per_hop && !big)
-            rc = atkb_pfb_hops(tbl_jobs(tb), tbl_carry(tb, p->max_nel), (int)nel, (int)m, p->d_counters, stream);
+            rc = atkb_pfb_hops(tbl_jobs(tb), tbl_carry(tb, p->max_nel), (int)nel, (int)m, (int)p->nchan, p->d_counters,
+                               stream);
         else if ((from_params || cv->doff) && !big)   /* right after the table kernel */
             rc = atkb_pfb_launch_pdl(tbl_jobs(tb), tbl_tiles(tb, p->max_nel), tbl_carry(tb, p->max_nel),
                                      (int)nel, p->d_counters, p->grid < work ? p->grid : work,

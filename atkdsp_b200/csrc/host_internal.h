@@ -23,6 +23,13 @@ atkdsp_pfb *atkb_pfb_create_served(double fs, unsigned nchan, unsigned oversampl
 /* small calls of at most this many hops (over all elements) run one CTA per
  * hop; beyond it the tile kernel's throughput wins */
 #define ATKB_PER_HOP_MAX 1024
+/* a device call of one element and at most this many output points (hops x
+ * nchan) runs one CTA per hop too. Measured per call, tile kernel / per-hop
+ * kernel: nchan 1024, 2x, 16 taps 18.5 / 12.4 us at 128 hops and 20.2 / 22.5 at
+ * 256; nchan 256, 2x, 8 taps 14.4 / 9.7 at 512 hops and 14.4 / 16.5 at 1024;
+ * nchan 64, 2x, 16 taps 15.5 / 12.4 at 2048: the line lies at one wave of
+ * 2^17 points whatever the nchan. */
+#define ATKB_HOPS1_POINTS ((size_t)1 << 17)
 /* ... and write at most this many outputs straight into pinned host memory */
 #define ATKB_DIRECT_OUT 2048
 

@@ -226,8 +226,11 @@ int  atkb_pfb_debug_build(void);
 /* small calls: one CTA per hop of njobs jobs of m hops each (the bank a
  * power of two 16..1024 on the fast plan, atkb_pfb_hops_ok), then one CTA per
  * carry; the same outputs and fault word as atkb_pfb_launch */
-int  atkb_pfb_hops(const atkb_job *d_jobs, const atkb_carry *d_carry, int njobs, int m, int *d_counters,
+int  atkb_pfb_hops(const atkb_job *d_jobs, const atkb_carry *d_carry, int njobs, int m, int nchan, int *d_counters,
                    void *stream);
+/* the same for one job given in host memory (passed as launch parameters:
+ * no table in device memory; the constants of doff derived in the kernel) */
+int  atkb_pfb_hops1(const atkb_job *J, const atkb_carry *C, int m, int nchan, int *d_counters, void *stream);
 int  atkb_pfb_hops_ok(const atkb_bank *B);
 /* the int16 constants of nel device jobs and carries whose doff is set, from
  * that device-held offset (after the table upload, before the tile kernel) */
@@ -343,7 +346,7 @@ int  atkb_osx_carry(const void *state, long long state_stride, const void *const
  * frames f < `frames` of n = 2^logn samples at in + f*hop (device cf32),
  * windowed by win (device, n floats, or NULL), transformed with the n-point
  * table tw; nblk CTAs take `per` consecutive frames each into `part`
- * (nblk lines: float for modes 0/1/2, 4 double planes for mode 3), then the
+ * (nblk lines of n doubles: one for modes 0/1/2, 4 planes for mode 3), then the
  * merged line goes to o0 (modes 0/1/2: max / min / average detector, dB) or
  * o0..o3 (mode 3: max / avg / min dB and kurtosis; NULL skips one). */
 #define ATKB_SPEC_NMAX 4096

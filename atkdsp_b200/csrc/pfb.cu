@@ -51,99 +51,7 @@
 
 namespace {
 
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-/* multiply by -i */
-__device__ __forceinline__ double2 cmi(double2 a) { return make_double2(a.y, -a.x); }
-
-/* the reference's rotation / cal product: one rounding per multiply and add */
-__device__ __forceinline__ double2 cmul_rn(double2 a, double2 b) {
-    return make_double2(__dsub_rn(__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y)),
-                        __dadd_rn(__dmul_rn(a.x, b.y), __dmul_rn(a.y, b.x)));
-}
-
-#define C16_1 0.92387953251128675613   /* cos(pi/8) */
-#define S16_1 0.38268343236508977173   /* sin(pi/8) */
-#define SQH   0.70710678118654752440   /* sqrt(1/2) */
-
-/* forward DFTs, e^{-2 pi i nk/R} */
-__device__ __forceinline__ void dft2(double2 &a, double2 &b) {
-    const double2 t = a;
-    a = cadd(t, b);
-    b = csub(t, b);
-}
-
-__device__ __forceinline__ void dft4(double2 &v0, double2 &v1, double2 &v2, double2 &v3) {
-    const double2 t0 = cadd(v0, v2), t1 = csub(v0, v2);
-    const double2 t2 = cadd(v1, v3), t3 = cmi(csub(v1, v3));
-    v0 = cadd(t0, t2);
-    v2 = csub(t0, t2);
-    v1 = cadd(t1, t3);
-    v3 = csub(t1, t3);
-}
-
-__device__ __forceinline__ void dft8(double2 *v) {
-    /* n = 2 n1 + n2, k = k1 + 4 k2 */
-    double2 a0 = v[0], a1 = v[2], a2 = v[4], a3 = v[6];
-    double2 b0 = v[1], b1 = v[3], b2 = v[5], b3 = v[7];
-    dft4(a0, a1, a2, a3);
-    dft4(b0, b1, b2, b3);
-    b1 = make_double2(SQH * (b1.x + b1.y), SQH * (b1.y - b1.x));      /* W8^1 */
-    b2 = cmi(b2);                                                     /* W8^2 */
-    b3 = make_double2(SQH * (b3.y - b3.x), -SQH * (b3.x + b3.y));     /* W8^3 */
-    v[0] = cadd(a0, b0); v[4] = csub(a0, b0);
-    v[1] = cadd(a1, b1); v[5] = csub(a1, b1);
-    v[2] = cadd(a2, b2); v[6] = csub(a2, b2);
-    v[3] = cadd(a3, b3); v[7] = csub(a3, b3);
-}
-
-__device__ __forceinline__ void dft16(double2 *v) {
-    /* n = 4 n1 + n2, k = k1 + 4 k2: radix-4 columns, W16^(n2 k1), radix-4
-     * rows, all in place; the rows leave y[k1 + 4 k2] at v[4 k1 + k2], and a
-     * final renaming (free once unrolled) restores natural order */
-#pragma unroll
-    for (int n2 = 0; n2 < 4; ++n2) dft4(v[n2], v[4 + n2], v[8 + n2], v[12 + n2]);
-    v[4 * 1 + 1] = cmul(v[4 * 1 + 1], make_double2(C16_1, -S16_1));
-    v[4 * 2 + 1] = cmul(v[4 * 2 + 1], make_double2(SQH, -SQH));
-    v[4 * 3 + 1] = cmul(v[4 * 3 + 1], make_double2(S16_1, -C16_1));
-    v[4 * 1 + 2] = cmul(v[4 * 1 + 2], make_double2(SQH, -SQH));
-    v[4 * 2 + 2] = cmi(v[4 * 2 + 2]);
-    v[4 * 3 + 2] = cmul(v[4 * 3 + 2], make_double2(-SQH, -SQH));
-    v[4 * 1 + 3] = cmul(v[4 * 1 + 3], make_double2(S16_1, -C16_1));
-    v[4 * 2 + 3] = cmul(v[4 * 2 + 3], make_double2(-SQH, -SQH));
-    v[4 * 3 + 3] = cmul(v[4 * 3 + 3], make_double2(-C16_1, S16_1));
-#pragma unroll
-    for (int k1 = 0; k1 < 4; ++k1) dft4(v[4 * k1], v[4 * k1 + 1], v[4 * k1 + 2], v[4 * k1 + 3]);
-    /* transpose the 4x4 index grid */
-    double2 t;
-    t = v[1]; v[1] = v[4]; v[4] = t;
-    t = v[2]; v[2] = v[8]; v[8] = t;
-    t = v[3]; v[3] = v[12]; v[12] = t;
-    t = v[6]; v[6] = v[9]; v[9] = t;
-    t = v[7]; v[7] = v[13]; v[13] = t;
-    t = v[11]; v[11] = v[14]; v[14] = t;
-}
-
-__device__ __forceinline__ void dft3(double2 &a, double2 &b, double2 &c) {
-    const double S3 = 0.86602540378443864676;   /* sin(2 pi / 3) */
-    const double2 s = cadd(b, c), d = csub(b, c);
-    const double2 m = make_double2(a.x - 0.5 * s.x, a.y - 0.5 * s.y);
-    const double2 r = make_double2(S3 * d.y, -S3 * d.x);  /* -i sin(2pi/3) (b - c) */
-    a = cadd(a, s);
-    b = cadd(m, r);
-    c = csub(m, r);
-}
-
-template <int R>
-__device__ __forceinline__ void dftR(double2 *v) {
-    if (R == 2) dft2(v[0], v[1]);
-    else if (R == 4) dft4(v[0], v[1], v[2], v[3]);
-    else if (R == 8) dft8(v);
-    else if (R == 16) dft16(v);
-}
+#include "pfb_dev.cuh"
 
 /* Per-thread index checks of the debug build (ATKB_DEBUG_BOUNDS): an index
  * outside its buffer sets a bit of g_atkb_debug_fault and the access is
@@ -160,37 +68,6 @@ __device__ __forceinline__ bool idx_ok(bool ok) {
 #define IDX_OK(c) true
 #endif
 
-/* one element of the stream s = state[0, head) ++ in[0, ...) */
-/* int16 I/Q -> cf32 exactly as the unpack front end does, (float(v) - c) * k
- * with rounded operations (reference src/convert.c:64-73), in the fused form
- * the host prepares: nc = -(c * k) with k a power of two, one rounding */
-__device__ __forceinline__ float2 conv16(short2 v, float ncre, float ncim, float k) {
-    return make_float2(__fmaf_rn((float)v.x, k, ncre), __fmaf_rn((float)v.y, k, ncim));
-}
-
-/* one element of the stream s = state[0, head) ++ in[0, ...); `in` is cf32 or
- * raw int16 I/Q converted on the fly */
-struct Src {
-    const float2 *st;
-    const void *in;
-    long long head;
-    int kind;
-    float cre, cim, k;
-    __device__ __forceinline__ float2 at(long long i) const {
-        if (i < head) return __ldg(st + i);
-        if (kind) return conv16(__ldg((const short2 *)in + (i - head)), cre, cim, k);
-        return __ldg((const float2 *)in + (i - head));
-    }
-};
-
-/* The int16 constants from an offset held in device memory (a job's or a
- * carry's doff): atkb_job_conv's -((off / k) * k), off the double rounded to
- * float, by the same IEEE float operations as the host. */
-__device__ __forceinline__ void doff_consts(const double *doff, float k, float &cre, float &cim) {
-    cre = -__fmul_rn(__fdiv_rn(__double2float_rn(__ldg(doff)), k), k);
-    cim = -__fmul_rn(__fdiv_rn(__double2float_rn(__ldg(doff + 1)), k), k);
-}
-
 /* ---- fast path: nchan = 2^n, 16 <= nchan <= 4096 ------------------------- */
 /* Shared-memory index swizzle for the 16-byte complex doubles: the low LOGP
  * index bits are XORed with the next LOGP. The first pass stores at a stride
@@ -199,28 +76,6 @@ __device__ __forceinline__ void doff_consts(const double *doff, float k, float &
  * stay conflict-free too (a XOR with a per-block constant permutes the
  * slots). */
 __device__ __forceinline__ int SW(int i) { return i ^ ((i >> LOGP) & (PTS - 1)); }
-
-/* the twiddles of one butterfly, w[r] = W^(r k) for r = 1 .. R-1, from the
- * one table entry w1 = W^k: squares and products (each power carries at most
- * two double roundings more than a table entry, ~1e-16 relative) instead of
- * R-1 table loads, so a pass reads Ns table entries, not (R-1)*Ns */
-__device__ __forceinline__ double2 csq(double2 a) {
-    return make_double2(a.x * a.x - a.y * a.y, 2.0 * a.x * a.y);
-}
-template <int R>
-__device__ __forceinline__ void tw_powers(double2 w1, double2 *w) {
-    w[1] = w1;
-    if constexpr (R > 2) {
-        w[2] = csq(w1);
-        w[3] = cmul(w[2], w1);
-    }
-    if constexpr (R > 4) {
-        w[4] = csq(w[2]);
-        w[5] = cmul(w[4], w1);
-        w[6] = csq(w[3]);
-        w[7] = cmul(w[4], w[3]);
-    }
-}
 
 /* Barrier over the G consecutive threads that share a hop group (G a power of
  * two): a warp sync up to 32 threads, a named barrier (ids 1..NT/G) up to
@@ -286,19 +141,6 @@ __device__ __forceinline__ void pass_c(double2 *sm, const double2 *__restrict__ 
         for (int r = 0; r < R; ++r) sm[SW(dst[u] + r * NS)] = v[u][r];
     }
     group_sync<G>();
-}
-
-/* Rotation to input sample 0 and cal for bin kb of a hop whose (b + 1) mod os
- * is s, then one rounding to float (reference src/channelizer.c:270-292). */
-__device__ __forceinline__ float2 finish_bin(double2 X, int kb, int s, int M, int os, int hop,
-                                             bool os_pow2, const double2 *twd, const float2 *cal) {
-    const int jr = os_pow2 ? ((kb * s) & (os - 1)) : ((kb * s) % os);
-    X = cmul_rn(X, __ldg(twd + (jr ? M - jr * hop : 0)));
-    if (cal) {
-        const float2 c = __ldg(cal + kb);
-        X = cmul_rn(X, make_double2((double)c.x, (double)c.y));
-    }
-    return make_float2(__double2float_rn(X.x), __double2float_rn(X.y));
 }
 
 /* The last Stockham pass fused with the epilogue: after the butterflies every
@@ -1262,26 +1104,6 @@ __device__ __forceinline__ void fetch_tile(const atkb_job *__restrict__ jobs, co
     if (lane == 0) s_local[slot] = tile - tile_start[lo];
 }
 
-/* dst[0, len) = s[from, from + len), eight loads in flight per thread before
- * their stores (a load-store loop would wait one memory round trip per
- * step: the compiler cannot tell dst from the sources) */
-template <int T>
-__device__ __forceinline__ void carry_copy(const Src &src, float2 *dst, long long from, long long len) {
-    for (long long i0 = threadIdx.x; i0 < len; i0 += 8LL * T) {
-        float2 v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const long long i = i0 + (long long)u * T;
-            if (i < len) v[u] = src.at(from + i);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const long long i = i0 + (long long)u * T;
-            if (i < len) dst[i] = v[u];
-        }
-    }
-}
-
 #ifndef ATKB_TILE_MINB
 #define ATKB_TILE_MINB (PTS == 8 ? 2 : 2)
 #endif
@@ -1502,168 +1324,6 @@ big_out_kernel(const double2 *__restrict__ X, const atkb_job J, const double2 *_
 }
 
 
-/* ---- small calls: one CTA per hop ------------------------------------------
- * A host call of a few thousand samples completes a few dozen hops; the tile
- * kernel would run them as one tile in one CTA, whose fold and passes take
- * ~20 us of latency. Here every hop of every job gets its own CTA of
- * HOPS_NT threads (power-of-two nchan 16..1024 on the fast plan), and the
- * jobs' state carries one CTA each after them:
- *   fold    thread per branch q, k ascending, a rounded multiply then a
- *           rounded add: the bits of every tile shape's fold;
- *   FFT     the bank's own plan, pass by pass between two shared-memory
- *           buffers: the first pass (radix plan.radix[0], Ns = 1) without
- *           twiddles, the others with tw_powers of the bank's per-pass table
- *           and cmul, the last fused with finish_bin -- the arithmetic of the
- *           tile kernel's passes, so the outputs equal the tile path's bits.
- * The uniform bounds checks are the tile kernel's (window, output, carry). */
-#define HOPS_NT 128
-#define HOPS_MAXM 1024
-
-template <int R>
-__device__ __forceinline__ void hop_pass(const double2 *__restrict__ src, double2 *__restrict__ dst, int M, int Ns,
-                                         const double2 *__restrict__ tw, bool first) {
-    const int MR = M / R;
-    for (int j = threadIdx.x; j < MR; j += HOPS_NT) {
-        const int k = j & (Ns - 1);
-        double2 v[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = src[j + r * MR];
-        if (!first) {
-            double2 w[R];
-            tw_powers<R>(__ldg(tw + k), w);
-#pragma unroll
-            for (int r = 1; r < R; ++r) v[r] = cmul(v[r], w[r]);
-        }
-        dftR<R>(v);
-        const int d = (j - k) * R + k;
-#pragma unroll
-        for (int r = 0; r < R; ++r) dst[d + r * Ns] = v[r];
-    }
-}
-
-template <int R>
-__device__ __forceinline__ void hop_pass_last(const double2 *__restrict__ src, int M, int Ns,
-                                              const double2 *__restrict__ tw, bool first, const atkb_bank &B,
-                                              const atkb_job &J, long long t) {
-    const int MR = M / R;                       /* == Ns */
-    const double2 *twd = (const double2 *)B.twd;
-    const float2 *cal = (const float2 *)J.cal;
-    float2 *out = (float2 *)J.out;
-    const int osm = B.os - 1;
-    const int s = (int)(J.b0 + t + 1) & osm;
-    for (int j = threadIdx.x; j < MR; j += HOPS_NT) {
-        double2 v[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = src[j + r * MR];
-        if (!first) {
-            double2 w[R];
-            tw_powers<R>(__ldg(tw + j), w);
-#pragma unroll
-            for (int r = 1; r < R; ++r) v[r] = cmul(v[r], w[r]);
-        }
-        dftR<R>(v);
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int kb = j + r * Ns;
-            out[(long long)kb * J.ldo + J.out_col + t] = finish_bin(v[r], kb, s, M, osm + 1, B.hop, true, twd, cal);
-        }
-    }
-}
-
-__global__ void __launch_bounds__(HOPS_NT)
-pfb_hops_kernel(const atkb_job *__restrict__ jobs, const atkb_carry *__restrict__ carries, int njobs, int m,
-                int *counters) {
-    __shared__ double2 buf[2][HOPS_MAXM];
-    __shared__ atkb_bank SB;
-    const int b = blockIdx.x;
-    if (b >= njobs * m) {                       /* a state carry */
-        const int ci = b - njobs * m;
-        if (ci >= njobs) return;
-        const atkb_carry &C = carries[ci];
-        const long long from = C.from, len = C.len;
-        if (from < 0 || len < 0 || from + len > C.nsrc || len > C.cap) {
-            if (threadIdx.x == 0) atomicOr((unsigned *)&counters[ATKB_FAULT_WORD], ATKB_FAULT_CARRY);
-            return;
-        }
-        const Src src{(const float2 *)C.state, C.in, C.head, C.in_kind, C.cre, C.cim, C.kscale};
-        float2 *dst = (float2 *)C.dst;
-        carry_copy<HOPS_NT>(src, dst, from, len);
-        return;
-    }
-    const atkb_job &J = jobs[b / m];
-    const long long t = b % m;
-    {
-        static_assert(sizeof(atkb_bank) % 4 == 0, "word copies");
-        const int *bs = (const int *)J.bank;
-        int *bd = (int *)&SB;
-        for (int w = threadIdx.x; w < (int)(sizeof(atkb_bank) / 4); w += HOPS_NT) bd[w] = bs[w];
-    }
-    __syncthreads();
-    const int M = SB.nchan;
-    /* uniform across the CTA: a shape this kernel does not run, a window past
-     * the job's samples or a column past the row stride skips the hop */
-    {
-        unsigned bad = 0;
-        if (t >= J.hops || t * SB.hop + SB.L > J.nsrc) bad |= ATKB_FAULT_WINDOW;
-        if (J.out_col + t + 1 > J.ldo) bad |= ATKB_FAULT_OUTPUT;
-        if (!SB.plan.fast || M > HOPS_MAXM || M < 16) bad |= ATKB_FAULT_INDEX;
-        for (int p = 0; p < SB.plan.npass; ++p)
-            if (SB.plan.radix[p] != 2 && SB.plan.radix[p] != 4 && SB.plan.radix[p] != 8) bad |= ATKB_FAULT_INDEX;
-        if (bad) {
-            if (threadIdx.x == 0) atomicOr((unsigned *)&counters[ATKB_FAULT_WORD], bad);
-            return;
-        }
-    }
-    /* the fold, one branch per thread and step, eight taps' loads in flight */
-    {
-        const Src src{(const float2 *)J.state, J.in, J.head, J.in_kind, J.cre, J.cim, J.kscale};
-        const float *taps = SB.taps;
-        const int K = SB.K;
-        const long long base = t * SB.hop;
-        for (int q = threadIdx.x; q < M; q += HOPS_NT) {
-            float fr = -0.0f, fi = -0.0f;
-            for (int k0 = 0; k0 < K; k0 += 8) {
-                float h[8];
-                float2 x[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (k0 + u < K) {
-                        h[u] = __ldg(taps + (long long)(k0 + u) * M + q);
-                        x[u] = src.at(base + (long long)(k0 + u) * M + q);
-                    }
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (k0 + u < K) {
-                        fr = __fadd_rn(fr, __fmul_rn(h[u], x[u].x));
-                        fi = __fadd_rn(fi, __fmul_rn(h[u], x[u].y));
-                    }
-            }
-            buf[0][q] = make_double2((double)fr, (double)fi);
-        }
-    }
-    __syncthreads();
-    /* the plan's passes */
-    const double2 *wp = (const double2 *)SB.wpass;
-    int Ns = 1, cur = 0;
-    for (int p = 0; p < SB.plan.npass; ++p) {
-        const int R = SB.plan.radix[p];
-        const double2 *tw = wp + SB.plan.twoff[p];
-        const bool first = p == 0;
-        if (p == SB.plan.npass - 1) {
-            if (R == 8) hop_pass_last<8>(buf[cur], M, Ns, tw, first, SB, J, t);
-            else if (R == 4) hop_pass_last<4>(buf[cur], M, Ns, tw, first, SB, J, t);
-            else hop_pass_last<2>(buf[cur], M, Ns, tw, first, SB, J, t);
-        } else {
-            if (R == 8) hop_pass<8>(buf[cur], buf[cur ^ 1], M, Ns, tw, first);
-            else if (R == 4) hop_pass<4>(buf[cur], buf[cur ^ 1], M, Ns, tw, first);
-            else hop_pass<2>(buf[cur], buf[cur ^ 1], M, Ns, tw, first);
-            __syncthreads();
-            cur ^= 1;
-        }
-        Ns *= R;
-    }
-}
-
 }  // namespace
 
 extern "C" int atkb_pfb_max_smem(void) { return 200 * 1024; }
@@ -1801,25 +1461,6 @@ extern "C" int atkb_pfb_conv_from_offset(atkb_job *d_jobs, atkb_carry *d_carry, 
     if (nel < 1 || nel > 1024) return ATKB_E_ARG;
     conv_from_offset_kernel<<<1, nel, 0, (cudaStream_t)stream>>>(d_jobs, d_carry, nel);
     return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;
-}
-
-/* the small-call kernel: njobs jobs of m hops each, then their carries */
-extern "C" int atkb_pfb_hops(const atkb_job *d_jobs, const atkb_carry *d_carry, int njobs, int m, int *d_counters,
-                             void *stream) {
-    if (njobs < 1 || m < 0) return ATKB_E_ARG;
-    const long long grid = (long long)njobs * m + njobs;
-    if (grid > 0x7fffffffLL) return ATKB_E_ARG;
-    atkb_range_push("atkdsp small call");
-    pfb_hops_kernel<<<(unsigned)grid, HOPS_NT, 0, (cudaStream_t)stream>>>(d_jobs, d_carry, njobs, m, d_counters);
-    atkb_range_pop();
-    return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;
-}
-
-extern "C" int atkb_pfb_hops_ok(const atkb_bank *B) {
-    if (!B->plan.fast || B->plan.big || B->nchan < 16 || B->nchan > HOPS_MAXM) return 0;
-    for (int p = 0; p < B->plan.npass; ++p)
-        if (B->plan.radix[p] != 2 && B->plan.radix[p] != 4 && B->plan.radix[p] != 8) return 0;
-    return 1;
 }
 
 extern "C" unsigned atkb_pfb_debug_fault(void) {
