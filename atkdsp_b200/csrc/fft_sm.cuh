@@ -148,6 +148,66 @@ __device__ __forceinline__ void dft8(double2 *v, bool inv) {
     v[7] = d2sub(e[3], t3);
 }
 
+/* ---- butterflies with their twiddles in the multiply-adds --------------------
+ * R = 2^L points as L levels of radix-2 butterflies a, b -> a + w b, a - w b,
+ * six fused multiply-adds each (the second output is 2a minus the first); the
+ * input twiddles W^(r k) and the constant roots fold into each level's w, all
+ * from the one table entry w = W^k: 10.5 double operations a point at radix 8
+ * with the twiddles, where separate products and a split DFT take 13. X[k] is
+ * left at v[brev(k)]. Forward transforms only. */
+__device__ __forceinline__ void bfly2(double2 &a, double2 &b, double2 w) {
+    const double tx = __fma_rn(-w.y, b.y, __fma_rn(w.x, b.x, a.x));
+    const double ty = __fma_rn(w.y, b.x, __fma_rn(w.x, b.y, a.y));
+    b = make_double2(__fma_rn(2.0, a.x, -tx), __fma_rn(2.0, a.y, -ty));
+    a = make_double2(tx, ty);
+}
+/* the same with -i w */
+__device__ __forceinline__ void bfly2_mi(double2 &a, double2 &b, double2 w) {
+    bfly2(a, b, make_double2(w.y, -w.x));
+}
+__device__ __forceinline__ double2 mul_w8(double2 w) {
+    const double h = 0.70710678118654752440;
+    return make_double2(h * (w.x + w.y), h * (w.y - w.x));
+}
+template <int R>
+__device__ __forceinline__ void dft_tw(double2 *v, double2 w) {
+    if constexpr (R == 2) {
+        bfly2(v[0], v[1], w);
+    } else {
+        const double2 w2 = d2sq(w);
+        if constexpr (R == 4) {
+            bfly2(v[0], v[2], w2);
+            bfly2(v[1], v[3], w2);
+            bfly2(v[0], v[1], w);
+            bfly2_mi(v[2], v[3], w);
+        } else {
+            const double2 w4 = d2sq(w2), we = mul_w8(w);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) bfly2(v[r], v[r + 4], w4);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                bfly2(v[r], v[r + 2], w2);
+                bfly2_mi(v[4 + r], v[6 + r], w2);
+            }
+            bfly2(v[0], v[1], w);
+            bfly2_mi(v[2], v[3], w);
+            bfly2(v[4], v[5], we);
+            bfly2_mi(v[6], v[7], we);
+        }
+    }
+}
+template <int R>
+__host__ __device__ constexpr int brev(int k) {
+    return R == 2 ? k : R == 4 ? (k & 1) * 2 + (k >> 1) : (k & 1) * 4 + (k & 2) + (k >> 2);
+}
+/* sw of swz, with which point STEP * r past the one at byte offset a (whose
+ * index has no bits there) is one XOR away, plus a constant above bit 5 */
+template <int STEP>
+__device__ __forceinline__ double2 &swz_at(double2 *sm, int a, int r) {
+    const int lo = (STEP * r) & 63, hi = (STEP * r) & ~63;
+    return *(double2 *)((char *)sm + (a ^ ((lo ^ ((lo >> 3) & 7)) * 16)) + hi * 16);
+}
+
 /* One transform of n = 2^logn points (8 <= n <= 8*NTH) in the swizzled
  * layout by NTH threads, natural order in and out: radix-8 Stockham passes,
  * then one radix-4 or radix-2 pass for the bits left. A butterfly's

@@ -63,7 +63,11 @@ static ptrdiff_t spec_run(atkdsp_gpu_spectrum *p, int mode, const atkdsp_cf32 *d
     if (hop == 0 || hop > n) hop = n;
     if (n_samples < n) return 0;
     const long long frames = (long long)((n_samples - n) / hop + 1);
-    long long nblk = frames < p->maxblk ? frames : p->maxblk;
+    /* one wave: a CTA per SM for the statistics, two for a single line, each
+     * working on 4096/n frames at a time */
+    const long long at_once = (long long)(ATKB_SPEC_NMAX / n), most = mode == 3 ? p->maxblk / 2 : p->maxblk;
+    long long nblk = (frames + at_once - 1) / at_once;
+    if (nblk > most) nblk = most;
     const long long per = (frames + nblk - 1) / nblk;
     nblk = (frames + per - 1) / per;
     const int rc = atkb_spec_launch(mode, d_in, frames, (long long)hop, p->logn, d_window, p->d_tw, (int)nblk,
