@@ -608,7 +608,7 @@ atkdsp_pfb *atkb_pfb_create_internal(double fs, unsigned nchan, unsigned oversam
     if (rc == ATKB_OK) rc = atkb_memset(p->d_counters, 0, ATKB_NCOUNTERS * sizeof(int), p->stream);
     if (rc == ATKB_OK) rc = atkb_stream_sync(p->stream);
     if (rc != ATKB_OK) { atkdsp_pfb_destroy(p); return NULL; }
-    p->grid = atkb_pfb_grid(p->dev, p->bank.smem_bytes);
+    p->grid = atkb_pfb_grid(p->dev, p->bank.smem_bytes, &p->bank);
     if (p->grid < 1) { atkdsp_pfb_destroy(p); return NULL; }
     p->lc = 0;
     p->b = 0;
@@ -830,7 +830,7 @@ static int run_step_up(atkdsp_pfb *p, unsigned nel, const void *const *ins, size
     }
     T[nel] = (int)nel * tiles;
     /* one job of few points: one CTA per hop, the job in the launch's parameters */
-    if (nel == 1 && !up_extra && !J[0].w2 && m * p->nchan <= ATKB_HOPS1_POINTS && atkb_pfb_hops_ok(&p->bank)) {
+    if (nel == 1 && !up_extra && !J[0].w2 && m <= ATKB_HOPS1_MAX && m * p->nchan <= ATKB_HOPS1_POINTS && atkb_pfb_hops_ok(&p->bank)) {
         rc = atkb_pfb_hops1(&J[0], &C[0], (int)m, (int)p->nchan, p->d_counters, stream);
         if (rc != ATKB_OK) return rc;
         p->cur = (int)nxt;
@@ -881,11 +881,11 @@ static int run_step_up(atkdsp_pfb *p, unsigned nel, const void *const *ins, size
         else if ((from_params || cv->doff) && !big)   /* right after the table kernel */
             rc = atkb_pfb_launch_pdl(tbl_jobs(tb), tbl_tiles(tb, p->max_nel), tbl_carry(tb, p->max_nel),
                                      (int)nel, p->d_counters, p->grid < work ? p->grid : work,
-                                     p->bank.smem_bytes, stream);
+                                     p->bank.smem_bytes, &p->bank, stream);
         else
             rc = atkb_pfb_launch(tbl_jobs(tb), tbl_tiles(tb, p->max_nel),
                                  tbl_carry(tb, p->max_nel), (int)nel, p->d_counters,
-                                 p->grid < work ? p->grid : work, p->bank.smem_bytes, stream);
+                                 p->grid < work ? p->grid : work, p->bank.smem_bytes, &p->bank, stream);
         if (rc != ATKB_OK) return rc;
     }
     p->cur = (int)nxt;
@@ -1565,6 +1565,7 @@ struct atkdsp_gpu_batch {
     int *d_counters;
     int grid, smem;
     void *tk[2];                  /* timing events around the tile kernel */
+    const atkb_bank *bank;        /* the one bank of every handle, or NULL */
 };
 
 ATKDSP_API void atkdsp_gpu_batch_destroy(atkdsp_gpu_batch *b) {
@@ -1601,6 +1602,8 @@ ATKDSP_API atkdsp_gpu_batch *atkdsp_gpu_batch_create(atkdsp_pfb *const *handles,
         b->h[i] = handles[i];
         if (handles[i]->bank.smem_bytes > b->smem) b->smem = handles[i]->bank.smem_bytes;
     }
+    for (i = 1; i < count && handles[i]->be == handles[0]->be; ++i) {}
+    if (i == count) b->bank = &handles[0]->be->bank;
     atkb_set_device(b->dev);
     b->tbl_bytes = tables_bytes(count);
     int rc = atkb_stream_create(&b->stream);
@@ -1614,7 +1617,7 @@ ATKDSP_API atkdsp_gpu_batch *atkdsp_gpu_batch_create(atkdsp_pfb *const *handles,
     if (rc == ATKB_OK) rc = atkb_memset(b->d_counters, 0, ATKB_NCOUNTERS * sizeof(int), b->stream);
     if (rc == ATKB_OK) rc = atkb_stream_sync(b->stream);
     if (rc != ATKB_OK) { atkdsp_gpu_batch_destroy(b); return NULL; }
-    b->grid = atkb_pfb_grid(b->dev, b->smem);
+    b->grid = atkb_pfb_grid(b->dev, b->smem, b->bank);
     return b;
 }
 
@@ -1649,7 +1652,7 @@ static int batch_enqueue(atkdsp_gpu_batch *b, int slot, void *stream) {
     if (rc == ATKB_OK)
         rc = atkb_pfb_launch(tbl_jobs(b->d_tables), tbl_tiles(b->d_tables, b->count),
                              tbl_carry(b->d_tables, b->count), (int)b->count, b->d_counters, b->grid,
-                             b->smem, stream);
+                             b->smem, b->bank, stream);
     if (rc == ATKB_OK) rc = atkb_event_record_node(b->tk[1], stream);
     return rc;
 }

@@ -28,8 +28,10 @@ atkdsp_pfb *atkb_pfb_create_served(double fs, unsigned nchan, unsigned oversampl
  * kernel: nchan 1024, 2x, 16 taps 18.5 / 12.4 us at 128 hops and 20.2 / 22.5 at
  * 256; nchan 256, 2x, 8 taps 14.4 / 9.7 at 512 hops and 14.4 / 16.5 at 1024;
  * nchan 64, 2x, 16 taps 15.5 / 12.4 at 2048: the line lies at one wave of
- * 2^17 points whatever the nchan. */
+ * 2^17 points whatever the nchan; below nchan 64 at 2048 hops, where the CTAs
+ * themselves count (nchan 16, 2x, 12 taps, 8192 hops: 33 us, tile kernel 15). */
 #define ATKB_HOPS1_POINTS ((size_t)1 << 17)
+#define ATKB_HOPS1_MAX 2048
 /* ... and write at most this many outputs straight into pinned host memory */
 #define ATKB_DIRECT_OUT 2048
 

@@ -186,10 +186,12 @@ void atkb_range_pop(void);
 void atkb_graph_destroy(void *exec);
 
 /* filterbank --------------------------------------------------------------- */
-/* occupancy-derived number of CTAs for the persistent tile kernel */
-int  atkb_pfb_grid(int dev, int smem_bytes);
+/* occupancy-derived number of CTAs for the persistent tile kernel (of bank
+ * B's shape alone, or B NULL: of every shape), and its setup for launches */
+int  atkb_pfb_grid(int dev, int smem_bytes, const atkb_bank *B);
 int  atkb_pfb_max_smem(void);
-/* jobs / tile_start / carries / counters are DEVICE arrays; tile_start has
+/* B: the host copy of the one bank of every job, or NULL when the jobs may be
+ * of several. jobs / tile_start / carries / counters are DEVICE arrays; tile_start has
  * njobs + 1 entries, the last one the total tile count, read by the kernel
  * (so a captured graph can replay with new work). grid CTAs loop over the
  * tiles, then over the carries (one per job: it writes only the other state
@@ -198,7 +200,7 @@ int  atkb_pfb_max_smem(void);
  * leaves them zero again. */
 #define ATKB_NCOUNTERS 4
 int  atkb_pfb_launch(const atkb_job *d_jobs, const int *d_tile_start, const atkb_carry *d_carry,
-                     int njobs, int *d_counters, int grid, int smem_bytes, void *stream);
+                     int njobs, int *d_counters, int grid, int smem_bytes, const atkb_bank *B, void *stream);
 /* the same with the job count read from device memory (at most the given
  * maximum): a launch that serves a different set of streams each time can
  * be captured once */
@@ -209,7 +211,11 @@ int  atkb_pfb_launch_n(const atkb_job *d_jobs, const int *d_tile_start, const at
  * stream (which triggers early; the tile kernel waits for its completion
  * before reading the tables) */
 int  atkb_pfb_launch_pdl(const atkb_job *d_jobs, const int *d_tile_start, const atkb_carry *d_carry,
-                         int njobs, int *d_counters, int grid, int smem_bytes, void *stream);
+                         int njobs, int *d_counters, int grid, int smem_bytes, const atkb_bank *B,
+                         void *stream);
+/* the tile kernel of one tile key alone (pfb_one.cu), or NULL */
+const void *atkb_pfb_one(int key);
+unsigned atkb_pfb_one_fault(void);
 int  atkb_event_query(void *ev);        /* ATKB_OK when complete, 1 when pending */
 int  atkb_event_spin(void *ev);         /* wait for an event by polling it */
 /* large filterbanks (plan.big: nchan beyond one CTA's shared memory): hops

@@ -152,7 +152,7 @@ ATKDSP_API atkdsp_server *atkdsp_server_create(unsigned max_streams, size_t hbm_
     if (rc == ATKB_OK) rc = atkb_memset(s->d_counters, 0, ATKB_NCOUNTERS * sizeof(int), s->stream);
     if (rc == ATKB_OK) rc = atkb_stream_sync(s->stream);
     if (rc != ATKB_OK) { atkdsp_server_destroy(s); return NULL; }
-    s->grid = atkb_pfb_grid(s->dev, ATKB_FAST_SMEM_MAX);
+    s->grid = atkb_pfb_grid(s->dev, ATKB_FAST_SMEM_MAX, NULL);
     return s;
 }
 
