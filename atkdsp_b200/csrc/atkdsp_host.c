@@ -238,9 +238,12 @@ static int plan_fft(unsigned M, unsigned os, int want_pair, atkb_fft_plan *pl) {
         while (rem >= ATKB_PTS) { pl->radix[pl->npass++] = ATKB_PTS; rem /= ATKB_PTS; }
         if (rem > 1) pl->radix[pl->npass++] = (int)rem;
     } else {
+        /* radix 16 where every pass is a trip through HBM; inside a CTA radix 8
+         * keeps a butterfly in the registers of four CTAs per SM */
         unsigned rem = M, p;
-        while (rem % 16 == 0) { pl->radix[pl->npass++] = 16; rem /= 16; }
-        if (rem % 8 == 0) { pl->radix[pl->npass++] = 8; rem /= 8; }
+        const int large = M > MAX_GENERIC_NCHAN || is_pow2(M);
+        while (large && rem % 16 == 0) { pl->radix[pl->npass++] = 16; rem /= 16; }
+        while (rem % 8 == 0) { pl->radix[pl->npass++] = 8; rem /= 8; }
         if (rem % 4 == 0) { pl->radix[pl->npass++] = 4; rem /= 4; }
         if (rem % 2 == 0) { pl->radix[pl->npass++] = 2; rem /= 2; }
         for (p = 3; rem > 1; p += 2) {
@@ -829,9 +832,14 @@ static int run_step_up(atkdsp_pfb *p, unsigned nel, const void *const *ins, size
         job_conv(&J[e], &C[e], cv);
     }
     T[nel] = (int)nel * tiles;
-    /* one job of few points: one CTA per hop, the job in the launch's parameters */
-    if (nel == 1 && !up_extra && !J[0].w2 && m <= ATKB_HOPS1_MAX && m * p->nchan <= ATKB_HOPS1_POINTS && atkb_pfb_hops_ok(&p->bank)) {
-        rc = atkb_pfb_hops1(&J[0], &C[0], (int)m, (int)p->nchan, p->d_counters, stream);
+    /* one job on a generic bank, or of few points: one CTA per hop (or a few),
+     * the job in the launch's parameters */
+    const int generic = !p->bank.plan.fast && !big;
+    if (nel == 1 && !up_extra &&
+        (generic || (!J[0].w2 && m <= ATKB_HOPS1_MAX && m * p->nchan <= ATKB_HOPS1_POINTS &&
+                     atkb_pfb_hops_ok(&p->bank)))) {
+        rc = generic ? atkb_pfb_generic(&J[0], &C[0], 1, 1, (int)m, (int)p->nchan, p->d_counters, stream)
+                     : atkb_pfb_hops1(&J[0], &C[0], (int)m, (int)p->nchan, p->d_counters, stream);
         if (rc != ATKB_OK) return rc;
         p->cur = (int)nxt;
         p->lc = (unsigned)(p->lc + n - m * p->hop);
@@ -875,7 +883,10 @@ static int run_step_up(atkdsp_pfb *p, unsigned nel, const void *const *ins, size
         /* nel jobs: tile_start[nel] is their total (the kernel reads
          * tile_start[njobs]); the same launch copies the nel carries */
         const int work = (int)nel * tiles + (int)nel;
-        if (per_hop && !big)
+        if (generic)
+            rc = atkb_pfb_generic(tbl_jobs(tb), tbl_carry(tb, p->max_nel), 0, (int)nel, (int)m, (int)p->nchan,
+                                  p->d_counters, stream);
+        else if (per_hop && !big)
             rc = atkb_pfb_hops(tbl_jobs(tb), tbl_carry(tb, p->max_nel), (int)nel, (int)m, (int)p->nchan, p->d_counters,
                                stream);
         else if ((from_params || cv->doff) && !big)   /* right after the table kernel */
@@ -1565,6 +1576,7 @@ struct atkdsp_gpu_batch {
     int *d_counters;
     int grid, smem;
     void *tk[2];                  /* timing events around the tile kernel */
+    int generic_smem;             /* the generic banks' shared memory, 0: none */
     const atkb_bank *bank;        /* the one bank of every handle, or NULL */
 };
 
@@ -1600,7 +1612,9 @@ ATKDSP_API atkdsp_gpu_batch *atkdsp_gpu_batch_create(atkdsp_pfb *const *handles,
     if (!b->h) { free(b); return NULL; }
     for (i = 0; i < count; ++i) {
         b->h[i] = handles[i];
-        if (handles[i]->bank.smem_bytes > b->smem) b->smem = handles[i]->bank.smem_bytes;
+        /* generic banks' tiles run in a launch of their own */
+        int *most = handles[i]->bank.plan.fast ? &b->smem : &b->generic_smem;
+        if (handles[i]->bank.smem_bytes > *most) *most = handles[i]->bank.smem_bytes;
     }
     for (i = 1; i < count && handles[i]->be == handles[0]->be; ++i) {}
     if (i == count) b->bank = &handles[0]->be->bank;
@@ -1649,6 +1663,9 @@ ATKDSP_API float atkdsp_gpu_batch_kernel_ms(atkdsp_gpu_batch *b) {
 static int batch_enqueue(atkdsp_gpu_batch *b, int slot, void *stream) {
     int rc = atkb_h2d(b->d_tables, b->h_tables[slot], b->tbl_bytes, stream);
     if (rc == ATKB_OK) rc = atkb_event_record_node(b->tk[0], stream);
+    if (rc == ATKB_OK && b->generic_smem)
+        rc = atkb_pfb_generic_tiles(tbl_jobs(b->d_tables), tbl_tiles(b->d_tables, b->count), (int)b->count,
+                                    b->d_counters, b->generic_smem, stream);
     if (rc == ATKB_OK)
         rc = atkb_pfb_launch(tbl_jobs(b->d_tables), tbl_tiles(b->d_tables, b->count),
                              tbl_carry(b->d_tables, b->count), (int)b->count, b->d_counters, b->grid,

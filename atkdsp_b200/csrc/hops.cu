@@ -1,11 +1,13 @@
 /* Small calls of the filterbank: one CTA per hop. */
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <atomic>
 #include "internal.h"
 
 namespace {
 
 #include "pfb_dev.cuh"
+#include "pfb_generic.cuh"
 
 /* ---- small calls: one CTA per hop ------------------------------------------
  * A call of a few dozen to a few hundred hops cannot fill the tile kernel: its
@@ -200,6 +202,87 @@ pfb_hops1_kernel(const __grid_constant__ atkb_job J, const __grid_constant__ atk
     else hop_run<NTH>(J, cre, cim, blockIdx.x, hop_buf, SB, counters);
 }
 
+/* The same for a bank on the generic plan (any other nchan up to 6400): a CTA
+ * takes GH consecutive hops, as many as hold about 1024 points, of one job;
+ * every call of a single handle comes here, whatever its size, since no tile
+ * shares samples between hops anyway. One kernel for a table of jobs (m hops
+ * each) and for one job from the launch's parameters. Bound by the latency of
+ * the passes' shared-memory round trips: four CTAs of 256 threads per SM hide
+ * it (one CTA of 144 registers a thread: 121 us for nchan 1000, 2x, 12 taps,
+ * 500,003 samples; this one 37.5; the tile kernel's generic branch 94.0). */
+template <int NTH>
+__device__ __forceinline__ void generic_cta(const atkb_job &J, float cre, float cim, long long h0, int gh,
+                                            atkb_bank &SB, int *counters) {
+    extern __shared__ double2 hop_buf[];
+    const int *bs = (const int *)J.bank;
+    for (int w = threadIdx.x; w < (int)(sizeof(atkb_bank) / 4); w += NTH) ((int *)&SB)[w] = bs[w];
+    __syncthreads();
+    const long long left = J.hops - h0;
+    const int nvalid = (int)(left < gh ? left : gh);
+    unsigned bad = 0, dyn_smem;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_smem));
+    if (nvalid <= 0) return;
+    if ((h0 + nvalid - 1) * SB.hop + SB.L > J.nsrc) bad |= ATKB_FAULT_WINDOW;
+    if (J.out_col + h0 + nvalid > J.ldo) bad |= ATKB_FAULT_OUTPUT;
+    if (SB.plan.big || 32ll * nvalid * SB.nchan > (long long)dyn_smem) bad |= ATKB_FAULT_INDEX;
+    if (bad) {
+        if (threadIdx.x == 0) atomicOr((unsigned *)&counters[ATKB_FAULT_WORD], bad);
+        return;
+    }
+    generic_tile<NTH>(J, SB, cre, cim, h0, nvalid, hop_buf);
+}
+
+template <int NTH>
+__global__ void __launch_bounds__(NTH, 1024 / NTH)
+pfb_generic_kernel(const atkb_job *__restrict__ jobs, const atkb_carry *__restrict__ carries, int njobs, int groups,
+                   int gh, int *counters) {
+    __shared__ atkb_bank SB;
+    const int b = blockIdx.x;
+    if (b >= njobs * groups) {                  /* a state carry */
+        if (b - njobs * groups < njobs) {
+            const atkb_carry &C = carries[b - njobs * groups];
+            hop_carry<NTH>(C, C.cre, C.cim, counters);
+        }
+        return;
+    }
+    const atkb_job &J = jobs[b / groups];
+    generic_cta<NTH>(J, J.cre, J.cim, (long long)(b % groups) * gh, gh, SB, counters);
+}
+
+template <int NTH>
+__global__ void __launch_bounds__(NTH, 1024 / NTH)
+pfb_generic1_kernel(const __grid_constant__ atkb_job J, const __grid_constant__ atkb_carry C, int groups, int gh,
+                    int *counters) {
+    __shared__ atkb_bank SB;
+    float cre = J.cre, cim = J.cim;
+    if (J.doff) doff_consts(J.doff, J.kscale, cre, cim);
+    if ((int)blockIdx.x >= groups) hop_carry<NTH>(C, cre, cim, counters);
+    else generic_cta<NTH>(J, cre, cim, (long long)blockIdx.x * gh, gh, SB, counters);
+}
+
+/* the generic banks' tiles of a batch (tables as the tile kernel's, which
+ * passes them over and copies the carries): a fixed grid over all tiles, each
+ * CTA taking every gridDim-th, so that it can be captured once */
+__global__ void __launch_bounds__(256, 4)
+pfb_generic_tiles_kernel(const atkb_job *__restrict__ jobs, const int *__restrict__ tile_start, int njobs,
+                         int *counters) {
+    __shared__ atkb_bank SB;
+    const int total = tile_start[njobs];
+    for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
+        int lo = 0, hi = njobs - 1;             /* the last job whose first tile <= tile */
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (tile_start[mid] <= tile) lo = mid;
+            else hi = mid - 1;
+        }
+        const atkb_bank *B = jobs[lo].bank;
+        if (B->plan.fast || B->plan.big) continue;
+        __syncthreads();                        /* the last tile's reads of SB and of the points */
+        generic_cta<256>(jobs[lo], jobs[lo].cre, jobs[lo].cim, (long long)(tile - tile_start[lo]) * B->tile_hops,
+                         B->tile_hops, SB, counters);
+    }
+}
+
 }  // namespace
 
 /* threads of a hop's CTA: two branches each, 64 to 512 */
@@ -238,6 +321,66 @@ extern "C" int atkb_pfb_hops1(const atkb_job *J, const atkb_carry *C, int m, int
     }
     atkb_range_pop();
     return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;
+}
+
+/* hops a generic CTA takes: about 1024 points (nchan 24 43 hops, 1000 one);
+ * fewer when a launch of m hops would leave SMs idle */
+static int generic_hops(int nchan, long long m) {
+    long long gh = 1024 / nchan;
+    if (gh > (m + 295) / 296) gh = (m + 295) / 296;
+    return gh < 1 ? 1 : (int)gh;
+}
+
+template <int NTH>
+static int generic_launch(const atkb_job *jobs, const atkb_carry *carries, bool one, int njobs, int m, int nchan,
+                          int *d_counters, cudaStream_t st) {
+    /* the attributes are idempotent: concurrent first callers may both set them */
+    static std::atomic<bool> configured[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return ATKB_E_NODEV;
+    if (!configured[dev].load(std::memory_order_acquire)) {
+        const int most = 6400 * 32;
+        if (cudaFuncSetAttribute(pfb_generic_kernel<NTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess ||
+            cudaFuncSetAttribute(pfb_generic1_kernel<NTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess)
+            return ATKB_E_KERNEL;
+        configured[dev].store(true, std::memory_order_release);
+    }
+    const int gh = generic_hops(nchan, (long long)m * njobs), groups = (m + gh - 1) / gh;
+    const long long grid = (long long)njobs * groups + njobs;
+    if (grid > 0x7fffffffLL) return ATKB_E_ARG;
+    const size_t smem = (size_t)nchan * gh * 32;
+    if (one) pfb_generic1_kernel<NTH><<<(unsigned)grid, NTH, smem, st>>>(*jobs, *carries, groups, gh, d_counters);
+    else pfb_generic_kernel<NTH><<<(unsigned)grid, NTH, smem, st>>>(jobs, carries, njobs, groups, gh, d_counters);
+    return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;
+}
+
+extern "C" int atkb_pfb_generic_tiles(const atkb_job *d_jobs, const int *d_tile_start, int njobs, int *d_counters,
+                                      int smem_bytes, void *stream) {
+    static std::atomic<bool> configured[64];
+    int dev = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return ATKB_E_NODEV;
+    if (!configured[dev].load(std::memory_order_acquire)) {
+        if (cudaFuncSetAttribute(pfb_generic_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 6400 * 32) !=
+            cudaSuccess)
+            return ATKB_E_KERNEL;
+        configured[dev].store(true, std::memory_order_release);
+    }
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pfb_generic_tiles_kernel, 256, smem_bytes) !=
+        cudaSuccess || per_sm < 1)
+        per_sm = 1;
+    pfb_generic_tiles_kernel<<<per_sm * atkb_sm_count(dev), 256, smem_bytes, (cudaStream_t)stream>>>(
+        d_jobs, d_tile_start, njobs, d_counters);
+    return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;
+}
+
+extern "C" int atkb_pfb_generic(const atkb_job *jobs, const atkb_carry *carries, int one, int njobs, int m, int nchan,
+                                int *d_counters, void *stream) {
+    if (njobs < 1 || m < 0 || nchan < 2 || nchan > 6400) return ATKB_E_ARG;
+    atkb_range_push("atkdsp generic hops");
+    const int rc = nchan <= 1024 ? generic_launch<256>(jobs, carries, one != 0, njobs, m, nchan, d_counters, (cudaStream_t)stream)
+                                 : generic_launch<512>(jobs, carries, one != 0, njobs, m, nchan, d_counters, (cudaStream_t)stream);
+    atkb_range_pop();
+    return rc;
 }
 
 extern "C" int atkb_pfb_hops_ok(const atkb_bank *B) {

@@ -34,111 +34,13 @@
  *     load per butterfly, group barriers), the last pass fused with the
  *     rotation, cal, rounding and the transpose to channel-major; each
  *     channel gets a run of tile_hops consecutive outputs.
- *   - Generic path (any M >= 2): ping-pong shared buffers, mixed radix
- *     (2, 3, 4, 8, 16 butterflies, direct DFT for any other prime factor).
+ *   - Any other M up to 6400 has kernels of its own (hops.cu): here its tiles
+ *     are passed over and its carries copied.
  */
 #include <atomic>
 #include "pfb_kernel.cuh"
 
 namespace {
-
-/* ---- generic path: any nchan >= 2 ----------------------------------------- */
-__device__ void pass_generic(const double2 *src, double2 *dst, int M, int Ns, int R, int nh,
-                             const double2 *W) {
-    const int MR = M / R;
-    const int NsR = Ns * R;
-    const int stride = M / NsR;
-    for (int bi = threadIdx.x; bi < nh * MR; bi += NT) {
-        const int tt = bi / MR;
-        const int j = bi - tt * MR;
-        const int k = j % Ns;
-        const double2 *s = src + tt * M + j;
-        double2 *d = dst + tt * M + (j - k) * R + k;
-        if (R == 2 || R == 3 || R == 4 || R == 8 || R == 16) {
-            double2 v[16];
-            for (int r = 0; r < R; ++r) {
-                v[r] = s[r * MR];
-                if (r) v[r] = cmul(v[r], __ldg(W + r * k * stride));
-            }
-            if (R == 2) dft2(v[0], v[1]);
-            else if (R == 3) dft3(v[0], v[1], v[2]);
-            else if (R == 4) dft4(v[0], v[1], v[2], v[3]);
-            else if (R == 8) dft8(v);
-            else dft16(v);
-            for (int r = 0; r < R; ++r) d[r * Ns] = v[r];
-        } else {
-            /* direct DFT with the twiddle folded in: W_{NsR}^{r (k + o Ns)} */
-            for (int o = 0; o < R; ++o) {
-                double2 acc = make_double2(0.0, 0.0);
-                for (int r = 0; r < R; ++r) {
-                    const long long e = ((long long)r * (k + o * Ns)) % NsR;
-                    const double2 w = __ldg(W + e * stride);
-                    const double2 x = s[r * MR];
-                    acc.x += x.x * w.x - x.y * w.y;
-                    acc.y += x.x * w.y + x.y * w.x;
-                }
-                d[o * Ns] = acc;
-            }
-        }
-    }
-    __syncthreads();
-}
-
-__device__ void tile_generic(const atkb_job &J, const atkb_bank &B, long long h0, int nvalid,
-                             double2 *sm) {
-    const int M = B.nchan;
-    const int nh = B.tile_hops;
-    double2 *A = sm, *Bf = sm + (size_t)nh * M;
-    const Src src{(const float2 *)J.state, J.in, J.head, J.in_kind, J.cre, J.cim, J.kscale};
-    for (int e = threadIdx.x; e < nh * M; e += NT) {
-        const int tt = e / M;
-        const int q = e - tt * M;
-        double2 v = make_double2(0.0, 0.0);
-        if (tt < nvalid) {
-            const long long base = (h0 + tt) * (long long)B.hop + q;
-            float2 x = src.at(base);
-            float h = __ldg(B.taps + q);
-            float fr = __fmul_rn(h, x.x), fi = __fmul_rn(h, x.y);
-            for (int k = 1; k < B.K; ++k) {
-                h = __ldg(B.taps + (long long)k * M + q);
-                x = src.at(base + (long long)k * M);
-                fr = __fadd_rn(fr, __fmul_rn(h, x.x));
-                fi = __fadd_rn(fi, __fmul_rn(h, x.y));
-            }
-            v = make_double2((double)fr, (double)fi);
-        }
-        A[e] = v;
-    }
-    __syncthreads();
-    const double2 *W = (const double2 *)B.wfull;
-    int Ns = 1;
-    double2 *cur = A, *nxt = Bf;
-    for (int p = 0; p < B.plan.npass; ++p) {
-        const int R = B.plan.radix[p];
-        pass_generic(cur, nxt, M, Ns, R, nh, W);
-        Ns *= R;
-        double2 *t = cur; cur = nxt; nxt = t;
-    }
-    const double2 *twd = (const double2 *)B.twd;
-    const float2 *cal = (const float2 *)J.cal;
-    float2 *out = (float2 *)J.out;
-    const int os = B.os, hop = B.hop;
-    for (int e = threadIdx.x; e < nvalid * M; e += NT) {
-        const int kb = e / nvalid;
-        const int tt = e - kb * nvalid;
-        double2 X = cur[tt * M + kb];
-        const long long b = J.b0 + h0 + tt;
-        const int s = (int)((b + 1) % os);
-        const int jr = (int)(((long long)kb * s) % os);
-        X = cmul_rn(X, __ldg(twd + (jr ? M - jr * hop : 0)));
-        if (cal) {
-            const float2 c = __ldg(cal + kb);
-            X = cmul_rn(X, make_double2((double)c.x, (double)c.y));
-        }
-        out[(long long)kb * J.ldo + J.out_col + h0 + tt] =
-            make_float2(__double2float_rn(X.x), __double2float_rn(X.y));
-    }
-}
 
 struct AllShapes {
     static __device__ __forceinline__ void run(int key, const atkb_job &J, const atkb_bank &SB, long long h0,
@@ -150,8 +52,7 @@ struct AllShapes {
         T(12) T(16 + 12) T(32 + 12) T(48 + 12) EACH(80) EACH(96)
 #undef T
 #undef EACH
-        case -1: break;                      /* a tile to skip */
-        default: tile_generic(J, SB, h0, nvalid, sm); break;
+        default: break;
         }
     }
 };
