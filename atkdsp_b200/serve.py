@@ -10,10 +10,11 @@ block-latency percentiles. Device buffers are torch tensors.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 
 import torch
 
-from . import AtkDspError, FMT, _check, load
+from . import HERE, AtkDspError, FMT, _check, load
 
 __all__ = ["Server", "SimResult", "simulate"]
 
@@ -78,6 +79,21 @@ def _bind(lib):
     return lib
 
 
+def _load_native():
+    """The module that reads submit's arguments (csrc/py/submit.c), None where
+    it was built for another Python or not at all."""
+    spec = importlib.util.spec_from_file_location("_atkdsp_submit", HERE / "lib" / "_atkdsp_submit.so")
+    try:
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+    except ImportError:
+        return None
+    return mod
+
+
+_native = _load_native()
+
+
 class Server:
     def __init__(self, max_streams: int = 4096, hbm_reserve: int = 8 << 30, use_graph: bool = True):
         self._lib = _bind(load())
@@ -86,6 +102,7 @@ class Server:
             raise AtkDspError("server_create failed (no GPU or no memory)")
         self.max_streams = int(max_streams)
         self._done = (Done * (4 * self.max_streams))()
+        self._submit = C.cast(self._lib.atkdsp_server_submit, C.c_void_p).value
 
     def __del__(self):
         s = getattr(self, "_s", None)
@@ -104,6 +121,8 @@ class Server:
     def submit(self, sid: int, block: torch.Tensor, out: torch.Tensor, tag: int = 0,
                t_arrival: float = 0.0) -> int:
         """block: complex64 (cf32 stream) or int16 I/Q pairs (ci16 streams)."""
+        if _native is not None:
+            return _native.submit(self._submit, self._s or 0, torch.complex64, sid, block, out, tag, t_arrival)
         n = block.numel() if block.dtype == torch.complex64 else block.numel() // 2
         return int(self._lib.atkdsp_server_submit(self._s, int(sid), C.c_void_p(block.data_ptr()), n,
                                                   C.c_void_p(out.data_ptr()), out.numel(),
