@@ -27,34 +27,77 @@ namespace {
 constexpr double kLn10Over10 = 0.23025850929940458;   /* ln(10) / 10 */
 constexpr int kThreads = 256;
 
-__global__ void __launch_bounds__(kThreads) cfar_raw_kernel(const float *__restrict__ frames, int units,
-                                                            long long f0, int nf, long long nbins,
-                                                            double *__restrict__ raw, int ring) {
-    const long long total = (long long)nf * nbins;
-    for (long long e = (long long)blockIdx.x * kThreads + threadIdx.x; e < total;
-         e += (long long)gridDim.x * kThreads) {
-        const long long j = e / nbins, i = e - j * nbins;
-        double v = (double)frames[e];
-        if (units == 0) {
-            if (v < -300.0) v = -300.0;
-            v = exp(v * kLn10Over10);
-        } else if (v < 1e-30) {
-            v = 1e-30;
+/* The three kernels below take one bin and FR consecutive frames a thread:
+ * FR = 8 or 4 where that leaves two CTAs per SM, else 1 (a call of few cells
+ * is bound by the latency of one thread's chain). One frame a thread spent
+ * its time on 64-bit remainders of the ring (one per raw value read) and on
+ * the reference-cell table (one load of it per load of X): 9 + 13 + 25 us for
+ * a pass of 2^20 cells (4096 bins, CA over 32 cells, k 4). */
+__device__ __forceinline__ double linear_of(float x, int units) {
+    double v = (double)x;
+    if (units == 0) {
+        if (v < -300.0) v = -300.0;
+        v = exp(v * kLn10Over10);
+    } else if (v < 1e-30) {
+        v = 1e-30;
+    }
+    return v;
+}
+
+template <int FR>
+__global__ void __launch_bounds__(kThreads) cfar_raw_kernel(const float *__restrict__ frames, int units, int row0,
+                                                            int nf, long long nbins, double *__restrict__ raw,
+                                                            int ring) {
+    const long long i = (long long)blockIdx.x * kThreads + threadIdx.x;
+    if (i >= nbins) return;
+    for (int j0 = blockIdx.y * FR; j0 < nf; j0 += gridDim.y * FR) {
+        float x[FR];
+#pragma unroll
+        for (int u = 0; u < FR; ++u)
+            if (j0 + u < nf) x[u] = __ldg(frames + (long long)(j0 + u) * nbins + i);
+        int row = (int)(((long long)row0 + j0) % ring);
+#pragma unroll
+        for (int u = 0; u < FR; ++u) {
+            if (j0 + u < nf) raw[(long long)row * nbins + i] = linear_of(x[u], units);
+            if (++row == ring) row = 0;
         }
-        raw[((f0 + j) % ring) * nbins + i] = v;
     }
 }
 
-/* X row of frame f: the mean of raw rows f-k+1 .. f, oldest first */
-__global__ void __launch_bounds__(kThreads) cfar_mean_kernel(const double *__restrict__ raw, int ring, long long f0,
-                                                             long long t0, long long nbins, int k,
+/* X row of each tested frame: the mean of its raw row and the k - 1 before,
+ * oldest first; row0: the ring row of the first tested frame's oldest. K > 0:
+ * k known, the FR frames' raw rows read once (K a power of two, so the
+ * product with 1 / K rounds as the quotient does); K = 0: any k, one frame. */
+template <int K, int FR>
+__global__ void __launch_bounds__(kThreads) cfar_mean_kernel(const double *__restrict__ raw, int ring, int row0,
+                                                             int ntest, long long nbins, int k,
                                                              double *__restrict__ X) {
     const long long i = (long long)blockIdx.x * kThreads + threadIdx.x;
-    const long long f = t0 + blockIdx.y;
+    const int j0 = blockIdx.y * FR;
     if (i >= nbins) return;
-    double s = 0.0;
-    for (int r = 0; r < k; ++r) s = __dadd_rn(s, raw[((f - k + 1 + r) % ring) * nbins + i]);
-    X[(f - f0) * nbins + i] = __ddiv_rn(s, (double)k);
+    int row = (int)(((long long)row0 + j0) % ring);
+    if constexpr (K > 0) {
+        double v[FR + K - 1];
+#pragma unroll
+        for (int u = 0; u < FR + K - 1; ++u) {
+            if (j0 + u < ntest + K - 1) v[u] = raw[(long long)row * nbins + i];
+            if (++row == ring) row = 0;
+        }
+#pragma unroll
+        for (int u = 0; u < FR; ++u) {
+            double s = 0.0;
+#pragma unroll
+            for (int r = 0; r < K; ++r) s = __dadd_rn(s, v[u + r]);
+            if (j0 + u < ntest) X[(long long)(j0 + u) * nbins + i] = __dmul_rn(s, 1.0 / K);
+        }
+    } else {
+        double s = 0.0;
+        for (int r = 0; r < k; ++r) {
+            s = __dadd_rn(s, raw[(long long)row * nbins + i]);
+            if (++row == ring) row = 0;
+        }
+        X[(long long)j0 * nbins + i] = __ddiv_rn(s, (double)k);
+    }
 }
 
 /* the k-th smallest (0-based) of a[0..n), NaN-free: Hoare's selection,
@@ -107,22 +150,16 @@ __device__ __forceinline__ void bitonic_sort(double (&v)[1 << LOGP]) {
     }
 }
 
-/* one testable bin's statistic, threshold and hit. OSMAX > 0: the OS
- * statistic over at most OSMAX cells: up to 32 sorted in registers (padded
- * with +inf, which sorts after every cell), more gathered into a local array
- * and selected. */
+/* one testable bin's OS statistic over at most OSMAX cells of the row Xr: up
+ * to 32 sorted in registers (padded with +inf, which sorts after every cell),
+ * more gathered into a local array and selected */
 template <int OSMAX>
-__device__ __forceinline__ bool cell_test(long long i, long long row, long long nbins, int mode, int n_ref, int N,
-                                          int os_k, double alpha, double alpha_ca, double et,
-                                          const uint8_t *__restrict__ sided, const int32_t *__restrict__ idx,
-                                          const double *__restrict__ X, double *__restrict__ noise,
-                                          double *__restrict__ thr) {
-    const double *Xr = X + row;
-    double Z, a = alpha, scale = et;
+__device__ __forceinline__ double os_stat(long long i, long long nbins, int N, int os_k,
+                                          const int32_t *__restrict__ idx, const double *__restrict__ Xr) {
+    bool has_nan = false;
     if constexpr (OSMAX == 32) {
         /* the os_k-th smallest; a NaN among the cells makes T NaN */
         double v[32];
-        bool has_nan = false;
 #pragma unroll
         for (int q = 0; q < 32; ++q) {
             v[q] = q < N ? Xr[idx[(long long)q * nbins + i]] : CUDART_INF;
@@ -135,42 +172,44 @@ __device__ __forceinline__ bool cell_test(long long i, long long row, long long 
 #pragma unroll
         for (int q = 0; q < 32; ++q)
             pick |= (unsigned long long)__double_as_longlong(v[q]) & (0ull - (unsigned long long)(q == os_k - 1));
-        Z = has_nan ? CUDART_NAN : __longlong_as_double((long long)pick);
-    } else if constexpr (OSMAX > 0) {
+        return has_nan ? CUDART_NAN : __longlong_as_double((long long)pick);
+    } else {
         double v[OSMAX];
-        bool has_nan = false;
         for (int q = 0; q < N; ++q) {
             v[q] = Xr[idx[(long long)q * nbins + i]];
             has_nan |= isnan(v[q]);
         }
-        Z = has_nan ? CUDART_NAN : select_kth(v, N, os_k - 1);
-    } else if ((mode == 2 || mode == 3) && sided[i]) {
-        double L = 0.0, R = 0.0;
-        for (int q = 0; q < n_ref; ++q) L = __dadd_rn(L, Xr[idx[(long long)q * nbins + i]]);
-        for (int q = n_ref; q < N; ++q) R = __dadd_rn(R, Xr[idx[(long long)q * nbins + i]]);
-        L = __ddiv_rn(L, (double)n_ref);
-        R = __ddiv_rn(R, (double)n_ref);
-        if (isnan(L) || isnan(R)) Z = CUDART_NAN;
-        else Z = mode == 2 ? (L > R ? L : R) : (L < R ? L : R);
-    } else {
-        double s = 0.0;
-        for (int q = 0; q < N; ++q) s = __dadd_rn(s, Xr[idx[(long long)q * nbins + i]]);
-        Z = __ddiv_rn(s, (double)N);
-        if (mode == 2 || mode == 3) {
-            a = alpha_ca;
-            scale = 1.0;
-        }
+        return has_nan ? CUDART_NAN : select_kth(v, N, os_k - 1);
     }
-    const double t = __dmul_rn(a, Z);
-    thr[row + i] = t;
-    noise[row + i] = __ddiv_rn(Z, scale);
-    return Xr[i] > t;
 }
 
-template <int OSMAX>
-__global__ void __launch_bounds__(kThreads) cfar_cell_kernel(long long f0, long long t0, long long nbins, int mode,
-                                                             int n_ref, int N, int os_k, double alpha,
-                                                             double alpha_ca, double et,
+/* s[f] = the sum over the reference cells q0 .. q1, in table order, of the
+ * rows Xr + f * nbins: one table entry and FR values a step, four steps'
+ * loads in flight */
+template <int FR>
+__device__ __forceinline__ void cell_sums(const double *const (&Xr)[FR], const int32_t *__restrict__ col,
+                                          long long nbins, int q0, int q1, double (&s)[FR]) {
+#pragma unroll
+    for (int f = 0; f < FR; ++f) s[f] = 0.0;
+#pragma unroll 4
+    for (int q = q0; q < q1; ++q) {
+        const int b = __ldg(col + (long long)q * nbins);
+#pragma unroll
+        for (int f = 0; f < FR; ++f) s[f] = __dadd_rn(s[f], Xr[f][b]);
+    }
+}
+
+/* s / n, by the exact reciprocal where n is a power of two (the same bits) */
+__device__ __forceinline__ double over(double s, int n) {
+    return (n & (n - 1)) == 0 ? __dmul_rn(s, 1.0 / (double)n) : __ddiv_rn(s, (double)n);
+}
+
+/* OSMAX 0: the statistics that are sums, FR frames a thread; else the OS
+ * statistic, FR = 1. X, noise, thr, hits and bits: rows of the first tested
+ * frame. */
+template <int OSMAX, int FR>
+__global__ void __launch_bounds__(kThreads) cfar_cell_kernel(int ntest, long long nbins, int mode, int n_ref, int N,
+                                                             int os_k, double alpha, double alpha_ca, double et,
                                                              const uint8_t *__restrict__ ok,
                                                              const uint8_t *__restrict__ sided,
                                                              const int32_t *__restrict__ idx,
@@ -179,44 +218,77 @@ __global__ void __launch_bounds__(kThreads) cfar_cell_kernel(long long f0, long 
                                                              uint8_t *__restrict__ hits, uint32_t *__restrict__ bits,
                                                              long long words) {
     const long long i = (long long)blockIdx.x * kThreads + threadIdx.x;
-    const long long f = t0 - f0 + blockIdx.y;
-    const long long row = f * nbins;
-    bool hit = false;
-    if (i < nbins && !ok[i]) {
-        noise[row + i] = CUDART_NAN;
-        thr[row + i] = CUDART_NAN;
-        hits[row + i] = 0;
-    } else if (i < nbins) {
-        hit = cell_test<OSMAX>(i, row, nbins, mode, n_ref, N, os_k, alpha, alpha_ca, et, sided, idx, X, noise, thr);
-        hits[row + i] = hit;
+    const int f0 = blockIdx.y * FR;
+    const bool in = i < nbins, test = in && ok[i];
+    double Z[FR], a = alpha, scale = et;
+    const double *Xr[FR];
+#pragma unroll
+    for (int f = 0; f < FR; ++f)            /* frames past the last repeat it */
+        Xr[f] = X + (long long)(f0 + f < ntest ? f0 + f : ntest - 1) * nbins;
+    if (test) {
+        if constexpr (OSMAX > 0) {
+#pragma unroll
+            for (int f = 0; f < FR; ++f) Z[f] = os_stat<OSMAX>(i, nbins, N, os_k, idx, Xr[f]);
+        } else if ((mode == 2 || mode == 3) && sided[i]) {
+            double L[FR], R[FR];
+            cell_sums<FR>(Xr, idx + i, nbins, 0, n_ref, L);
+            cell_sums<FR>(Xr, idx + i, nbins, n_ref, N, R);
+#pragma unroll
+            for (int f = 0; f < FR; ++f) {
+                const double l = over(L[f], n_ref), r = over(R[f], n_ref);
+                if (isnan(l) || isnan(r)) Z[f] = CUDART_NAN;
+                else Z[f] = mode == 2 ? (l > r ? l : r) : (l < r ? l : r);
+            }
+        } else {
+            cell_sums<FR>(Xr, idx + i, nbins, 0, N, Z);
+#pragma unroll
+            for (int f = 0; f < FR; ++f) Z[f] = over(Z[f], N);
+            if (mode == 2 || mode == 3) {
+                a = alpha_ca;
+                scale = 1.0;
+            }
+        }
     }
-    /* the row as a bitmask too: bin i is bit i % 32 of word i / 32 */
-    const unsigned m = __ballot_sync(0xffffffffu, hit);
-    if ((threadIdx.x & 31) == 0 && (i >> 5) < words) bits[f * words + (i >> 5)] = m;
+#pragma unroll
+    for (int f = 0; f < FR; ++f) {
+        if (f0 + f >= ntest) break;
+        const long long e = (long long)(f0 + f) * nbins + i;
+        bool hit = false;
+        if (test) {
+            const double t = __dmul_rn(a, Z[f]);
+            thr[e] = t;
+            noise[e] = scale == 1.0 ? Z[f] : __ddiv_rn(Z[f], scale);
+            hit = Xr[f][i] > t;
+        } else if (in) {
+            noise[e] = CUDART_NAN;
+            thr[e] = CUDART_NAN;
+        }
+        if (in) hits[e] = hit;
+        /* the row as a bitmask too: bin i is bit i % 32 of word i / 32 */
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if ((threadIdx.x & 31) == 0 && (i >> 5) < words) bits[(f0 + f) * words + (i >> 5)] = m;
+    }
 }
 
-
-
 /* a pass's rows at its columns: rows of X and noise (row r of X / noise to
- * row r of Xc / Nc), then nraw raw rows from frame rf0 on (to Rc) */
+ * row r of Xc / Nc), then nraw raw rows from ring row rf0 on (to Rc) */
 __global__ void __launch_bounds__(kThreads) cfar_gather_kernel(const double *__restrict__ X,
                                                                const double *__restrict__ noise, long long nbins,
                                                                int rows, const double *__restrict__ raw, int ring,
-                                                               long long rf0, int nraw,
-                                                               const int32_t *__restrict__ cols, int ncol,
-                                                               double *__restrict__ Xc, double *__restrict__ Nc,
-                                                               double *__restrict__ Rc) {
+                                                               int rf0, int nraw, const int32_t *__restrict__ cols,
+                                                               int ncol, double *__restrict__ Xc,
+                                                               double *__restrict__ Nc, double *__restrict__ Rc) {
     const long long total = (long long)(rows + nraw) * ncol;
     for (long long e = (long long)blockIdx.x * kThreads + threadIdx.x; e < total;
          e += (long long)gridDim.x * kThreads) {
-        const long long r = e / ncol, q = e - r * ncol;
+        const long long r = total <= 0xffffffffLL ? (unsigned)e / (unsigned)ncol : e / ncol, q = e - r * ncol;
         const long long b = cols[q];
         if (r < rows) {
             Xc[e] = X[r * nbins + b];
             Nc[e] = noise[r * nbins + b];
         } else {
-            const long long rr = r - rows;
-            Rc[rr * ncol + q] = raw[((rf0 + rr) % ring) * nbins + b];
+            const int rr = (int)(r - rows);
+            Rc[(long long)rr * ncol + q] = raw[(long long)(((unsigned)rf0 + (unsigned)rr) % (unsigned)ring) * nbins + b];
         }
     }
 }
@@ -228,11 +300,23 @@ int grid_for(long long work) {
 
 }  // namespace
 
+/* bins x (groups of fr frames), two CTAs on every SM: enough to take fr */
+static bool wide_enough(long long nbins, long long nf, int fr) {
+    return (nbins + kThreads - 1) / kThreads * (nf / fr) >= 2 * 148;
+}
+
 extern "C" int atkb_cfar_raw(const float *frames, int units, long long f0, int nf, long long nbins, double *raw,
                              int ring, void *stream) {
-    if (nf <= 0) return ATKB_OK;
-    cfar_raw_kernel<<<grid_for((long long)nf * nbins), kThreads, 0, (cudaStream_t)stream>>>(frames, units, f0, nf,
-                                                                                             nbins, raw, ring);
+    if (nf <= 0 || nbins <= 0) return ATKB_OK;
+    cudaStream_t s = (cudaStream_t)stream;
+    const unsigned bx = (unsigned)((nbins + kThreads - 1) / kThreads);
+    const int row0 = (int)(f0 % ring);
+    if (wide_enough(nbins, nf, 8))
+        cfar_raw_kernel<8><<<dim3(bx, (unsigned)((nf + 7) / 8 < 65535 ? (nf + 7) / 8 : 65535)), kThreads, 0, s>>>(
+            frames, units, row0, nf, nbins, raw, ring);
+    else
+        cfar_raw_kernel<1><<<dim3(bx, (unsigned)(nf < 65535 ? nf : 65535)), kThreads, 0, s>>>(frames, units, row0,
+                                                                                              nf, nbins, raw, ring);
     return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;
 }
 
@@ -241,26 +325,34 @@ extern "C" int atkb_cfar_test(const double *raw, int ring, long long f0, long lo
                               double et, const uint8_t *ok, const uint8_t *sided, const int32_t *idx, double *X,
                               double *noise, double *thr, uint8_t *hits, uint32_t *bits, long long words,
                               void *stream) {
-    const long long ntest = f0 + nf - t0;
+    const long long ntest = f0 + nf - t0, r0 = t0 - f0;
     if (ntest <= 0) return ATKB_OK;
     if (ntest > 65535 || nbins <= 0) return ATKB_E_ARG;
-    const dim3 grid((unsigned)((nbins + kThreads - 1) / kThreads), (unsigned)ntest);
+    const unsigned bx = (unsigned)((nbins + kThreads - 1) / kThreads);
+    const dim3 one(bx, (unsigned)ntest), four(bx, (unsigned)((ntest + 3) / 4)), eight(bx, (unsigned)((ntest + 7) / 8));
     cudaStream_t s = (cudaStream_t)stream;
-    cfar_mean_kernel<<<grid, kThreads, 0, s>>>(raw, ring, f0, t0, nbins, k, X);
-    if (mode != 1)
-        cfar_cell_kernel<0><<<grid, kThreads, 0, s>>>(f0, t0, nbins, mode, n_ref, n_cells, os_k, alpha, alpha_ca, et,
-                                                      ok, sided, idx, X, noise, thr, hits, bits, words);
-    else if (n_cells <= 32)
-        cfar_cell_kernel<32><<<grid, kThreads, 0, s>>>(f0, t0, nbins, mode, n_ref, n_cells, os_k, alpha, alpha_ca, et,
-                                                       ok, sided, idx, X, noise, thr, hits, bits, words);
-    else if (n_cells <= 64)
-        cfar_cell_kernel<64><<<grid, kThreads, 0, s>>>(f0, t0, nbins, mode, n_ref, n_cells, os_k, alpha, alpha_ca, et,
-                                                       ok, sided, idx, X, noise, thr, hits, bits, words);
-    else if (n_cells <= 512)
-        cfar_cell_kernel<512><<<grid, kThreads, 0, s>>>(f0, t0, nbins, mode, n_ref, n_cells, os_k, alpha, alpha_ca,
-                                                        et, ok, sided, idx, X, noise, thr, hits, bits, words);
-    else
-        return ATKB_E_ARG;
+    const int row0 = (int)((t0 - k + 1) % ring), n = (int)ntest;
+    X += r0 * nbins;
+    noise += r0 * nbins;
+    thr += r0 * nbins;
+    hits += r0 * nbins;
+    bits += r0 * words;
+    const bool w8 = wide_enough(nbins, ntest, 8);
+    if (k == 1 && w8) cfar_mean_kernel<1, 8><<<eight, kThreads, 0, s>>>(raw, ring, row0, n, nbins, k, X);
+    else if (k == 2 && w8) cfar_mean_kernel<2, 8><<<eight, kThreads, 0, s>>>(raw, ring, row0, n, nbins, k, X);
+    else if (k == 4 && w8) cfar_mean_kernel<4, 8><<<eight, kThreads, 0, s>>>(raw, ring, row0, n, nbins, k, X);
+    else if (k == 8 && w8) cfar_mean_kernel<8, 8><<<eight, kThreads, 0, s>>>(raw, ring, row0, n, nbins, k, X);
+    else cfar_mean_kernel<0, 1><<<one, kThreads, 0, s>>>(raw, ring, row0, n, nbins, k, X);
+#define CELLS(OSMAX, FR, GRID)                                                                                     \
+    cfar_cell_kernel<OSMAX, FR><<<GRID, kThreads, 0, s>>>(n, nbins, mode, n_ref, n_cells, os_k, alpha, alpha_ca,   \
+                                                          et, ok, sided, idx, X, noise, thr, hits, bits, words)
+    if (mode != 1 && wide_enough(nbins, ntest, 4)) CELLS(0, 4, four);
+    else if (mode != 1) CELLS(0, 1, one);
+    else if (n_cells <= 32) CELLS(32, 1, one);
+    else if (n_cells <= 64) CELLS(64, 1, one);
+    else if (n_cells <= 512) CELLS(512, 1, one);
+    else return ATKB_E_ARG;
+#undef CELLS
     return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;
 }
 
@@ -269,6 +361,6 @@ extern "C" int atkb_cfar_gather(const double *X, const double *noise, long long 
                                 double *Nc, double *Rc, void *stream) {
     if (ncol <= 0 || rows + nraw <= 0) return ATKB_OK;
     cfar_gather_kernel<<<grid_for((long long)(rows + nraw) * ncol), kThreads, 0, (cudaStream_t)stream>>>(
-        X, noise, nbins, rows, raw, ring, rf0, nraw, cols, ncol, Xc, Nc, Rc);
+        X, noise, nbins, rows, raw, ring, (int)(rf0 % ring), nraw, cols, ncol, Xc, Nc, Rc);
     return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;
 }

@@ -28,6 +28,7 @@
 /* frames per device pass: at most this many cells, and at most 4096 frames */
 #define CF_PASS_CELLS ((size_t)1 << 20)
 #define CF_PASS_FRAMES 4096
+#define CF_DIRECT_VALUES ((size_t)1 << 16)   /* a gather's results written straight to pinned memory */
 /* host buffers up to this size are pinned */
 #define CF_PINNED_MAX ((size_t)256 << 20)
 
@@ -551,8 +552,8 @@ ATKDSP_API void atkdsp_cfar_destroy(atkdsp_cfar *c) {
     free(c->beta);
     free(c->tracks);
     free(c->blobs);
-    free(c->last_X);
-    free(c->last_thr);
+    host_buf_free(c, c->last_X);
+    host_buf_free(c, c->last_thr);
     free(c->last_hits);
     free(c->ht);
     free(c->hd);
@@ -619,7 +620,7 @@ ATKDSP_API atkdsp_cfar *atkdsp_cfar_create(size_t nbins, const atkdsp_cfar_confi
     const size_t rrows = rows + (size_t)k - 1;     /* raw rows a pass's tracker reads */
     c->words = (nb + 31) / 32;
     const size_t W = c->words;
-    c->pinned = (2 * rows * W * 4 + 2 * rows * nb * 8 + (k > 1 ? rrows * nb * 8 : 0) + nb * 4) <= CF_PINNED_MAX;
+    c->pinned = (2 * rows * W * 4 + 2 * rows * nb * 8 + (k > 1 ? rrows * nb * 8 : 0) + nb * 20) <= CF_PINNED_MAX;
     c->next_id = 1;
     c->mask = (uint8_t *)calloc(nb, 1);
     c->ok = (uint8_t *)calloc(nb, 1);
@@ -627,8 +628,8 @@ ATKDSP_API atkdsp_cfar *atkdsp_cfar_create(size_t nbins, const atkdsp_cfar_confi
     c->beta = (double *)malloc((nb + 1) * sizeof(double));
     c->tracks = (cf_track *)calloc((size_t)c->cfg.max_tracks, sizeof(cf_track));
     c->blobs = (cf_blob *)calloc(nb, sizeof(cf_blob));
-    c->last_X = (double *)calloc(nb, sizeof(double));
-    c->last_thr = (double *)calloc(nb, sizeof(double));
+    c->last_X = (double *)host_buf(c, nb * sizeof(double));
+    c->last_thr = (double *)host_buf(c, nb * sizeof(double));
     c->last_hits = (uint8_t *)calloc(nb, 1);
     c->ht = (double *)calloc(ring, sizeof(double));
     c->hd = (double *)calloc(ring, sizeof(double));
@@ -1013,18 +1014,16 @@ static int pass_enqueue(atkdsp_cfar *c, const cf_pass *ps, const float *frames, 
         src = c->d_frames;
     }
     if (rc == ATKB_OK) rc = atkb_cfar_raw(src, units, F0, nf, (long long)nb, c->d_raw, c->ring, c->stream);
+    /* the caller's hit rows are the test's own output */
+    uint8_t *hits = d_hits_out ? d_hits_out + ps->done * nb : c->d_hits + hs;
     if (rc == ATKB_OK && j0 < nf)
         rc = atkb_cfar_test(c->d_raw, c->ring, F0, F0 + j0, nf, (long long)nb, k, c->cfg.mode, c->cfg.n_ref, c->N,
                             c->cfg.os_k, c->alpha, c->alpha_ca, c->et, c->d_ok, c->d_sided, c->d_idx, c->d_X + hs,
-                            c->d_noise + hs, c->d_thr + hs, c->d_hits + hs, c->d_bits + bs, (long long)W,
+                            c->d_noise + hs, c->d_thr + hs, hits, c->d_bits + bs, (long long)W,
                             c->stream);
-    if (rc == ATKB_OK && j0 < nf) {
-        const size_t off = (size_t)j0 * nb, rows = (size_t)(nf - j0) * nb;
+    if (rc == ATKB_OK && j0 < nf)
         rc = atkb_d2h(c->h_bits + bs + (size_t)j0 * W, c->d_bits + bs + (size_t)j0 * W,
                       (size_t)(nf - j0) * W * sizeof(uint32_t), c->stream);
-        if (rc == ATKB_OK && d_hits_out)
-            rc = atkb_d2d(d_hits_out + (ps->done + (size_t)j0) * nb, c->d_hits + hs + off, rows, c->stream);
-    }
     if (rc == ATKB_OK && d_hits_out && j0 > 0)
         rc = atkb_memset(d_hits_out + ps->done * nb, 0, (size_t)(j0 < nf ? j0 : nf) * nb, c->stream);
     if (rc == ATKB_OK) rc = atkb_event_record(c->ev_pass[set], c->stream);
@@ -1123,15 +1122,23 @@ static ptrdiff_t cfar_run(atkdsp_cfar *c, const float *frames, int on_device, in
             if (rc == ATKB_OK && c->ncol > 0) {
                 const int rows = cur.nf - j0, nraw = k > 1 ? rows + k - 1 : 0;
                 const size_t nc = (size_t)c->ncol;
+                /* few values: the gather writes the pinned rows itself (a pass
+                 * of 256 frames at 25 columns: one launch against three copies
+                 * behind it); many go by copies at the link's full rate */
+                const int direct = c->pinned && (size_t)(2 * rows + nraw) * nc <= CF_DIRECT_VALUES;
                 rc = atkb_h2d(c->d_cols, c->h_cols, nc * sizeof(int32_t), c->gstream);
                 if (rc == ATKB_OK)
                     rc = atkb_cfar_gather(c->d_X + hs + (size_t)j0 * nb, c->d_noise + hs + (size_t)j0 * nb,
                                           (long long)nb, rows, c->d_raw, c->ring, c->rc_f0, nraw, c->d_cols,
-                                          c->ncol, c->d_Xc, c->d_Nc, c->d_Rc, c->gstream);
-                if (rc == ATKB_OK) rc = atkb_d2h(c->h_Xc, c->d_Xc, (size_t)rows * nc * sizeof(double), c->gstream);
-                if (rc == ATKB_OK) rc = atkb_d2h(c->h_Nc, c->d_Nc, (size_t)rows * nc * sizeof(double), c->gstream);
-                if (rc == ATKB_OK && nraw)
-                    rc = atkb_d2h(c->h_Rc, c->d_Rc, (size_t)nraw * nc * sizeof(double), c->gstream);
+                                          c->ncol, direct ? c->h_Xc : c->d_Xc, direct ? c->h_Nc : c->d_Nc,
+                                          direct ? c->h_Rc : c->d_Rc, c->gstream);
+                if (rc == ATKB_OK && !direct) {
+                    rc = atkb_d2h(c->h_Xc, c->d_Xc, (size_t)rows * nc * sizeof(double), c->gstream);
+                    if (rc == ATKB_OK)
+                        rc = atkb_d2h(c->h_Nc, c->d_Nc, (size_t)rows * nc * sizeof(double), c->gstream);
+                    if (rc == ATKB_OK && nraw)
+                        rc = atkb_d2h(c->h_Rc, c->d_Rc, (size_t)nraw * nc * sizeof(double), c->gstream);
+                }
                 if (rc == ATKB_OK) rc = atkb_stream_sync(c->gstream);
             }
         }
