@@ -12,8 +12,9 @@
  * here every sum is double, reduced in a fixed order, so the results are
  * deterministic and at least as accurate.
  *
- * Work split inside a CTA: the upper triangle of the nel x nel matrix is cut
- * into TB x TB tiles (TB = 1, 2 or 4 by nel), and the threads into (tile, hop
+ * 2 to 8 elements: the FP64 matrix instruction (w12_mma_kernel). Otherwise
+ * the work split inside a CTA: the upper triangle of the nel x nel matrix is cut
+ * into TB x TB tiles (TB = 1 or 4 by nel), and the threads into (tile, hop
  * group) pairs: each thread keeps a tile's TB*TB sums in registers over its
  * share of the hops, so one hop's 2*TB loads feed TB*TB products (the old
  * one-pair-per-thread split loaded both operands for every product). The
@@ -241,6 +242,122 @@ __global__ void cov_reset_kernel(float2 *R, uint32_t *counts, int nel, int nchan
 }
 
 
+/* W1 / W2 of 2 to 8 elements through the FP64 matrix instruction (m8n8k4): a
+ * warp's lane holds one sample of four hops' 8 x 4 block, rows the elements,
+ * and that register is the A and the B fragment at once, so four hops' S is
+ *   Re += R R^T + I I^T,   Im += I R^T - R I^T
+ * in four instructions after one load and two conversions a lane. Arrays of at
+ * most NR = 4 (2) elements stack G = 8 / NR groups of four hops in the rows;
+ * the cross-group blocks of the product are not used. Each warp of a channel's
+ * CTA takes a run of hops; the warps' sums are added in warp order.
+ *
+ * The tile-per-thread kernel converts every sample three times for 8
+ * elements, spends a quarter of its passes on one hop in 85, and sums 85
+ * partials in 48 threads; this one is bound by the matrix unit's double rate
+ * (256 products a hop, 16 us) and the samples' trip from L2. Before and after,
+ * us: 8 elements x 2048 channels x 513 hops 88.3, 30.2; 8 x 256 x 4097 53.5,
+ * 26.9; 4 x 2048 x 513 76.1, 20.2; 2 x 1024 x 2000 23.9, 15.6. */
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+template <int NR>
+__global__ void __launch_bounds__(W_NT)
+w12_mma_kernel(const float2 *__restrict__ out, int nel, int nchan, long long m, const uint8_t *__restrict__ gate,
+               float2 *__restrict__ R, uint32_t *__restrict__ counts, float *__restrict__ pwr,
+               float *__restrict__ mean_pwr) {
+    constexpr int G = 8 / NR, STEP = 4 * G, U = 8;
+    __shared__ double part[W_NT / 32][2][64];
+    __shared__ double diag[8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int row = lane >> 2, el = row % NR;
+    const long long at = (row / NR) * 4 + (lane & 3);        /* the lane's hop of a step */
+    /* each warp's run: an equal share of the steps */
+    const long long steps = (m + STEP - 1) / STEP, share = (steps + warps - 1) / warps;
+    const long long s0 = (warp * share < steps ? warp * share : steps) * STEP;
+    long long s1 = s0 + share * STEP;
+    if (s1 > m) s1 = m;
+    for (int k = blockIdx.x; k < nchan; k += gridDim.x) {
+        const bool w1 = R && counts && (!gate || gate[k]);
+        const bool w2 = pwr || mean_pwr;
+        if (!w1 && !w2) continue;
+        const float2 *y = out + ((long long)(el < nel ? el : 0) * nchan + k) * m + at;
+        const long long end = el < nel ? s1 - at : 0;        /* y[i] is a sample of this run while i < end */
+        double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
+        for (long long i = s0; i < s1; i += U * STEP) {
+            float2 v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = i + u * STEP < end ? __ldg(y + i + u * STEP) : make_float2(0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const double x = (double)v[u].x, z = (double)v[u].y;
+                dmma(re, x, x);
+                if (w1) dmma(im, z, x);
+                dmma(re, z, z);
+                if (w1) dmma(im, -x, z);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            part[warp][0][row * 8 + (lane & 3) * 2 + c] = re[c];
+            part[warp][1][row * 8 + (lane & 3) * 2 + c] = im[c];
+        }
+        __syncthreads();
+        const int a = threadIdx.x / NR, b = threadIdx.x % NR;
+        if (threadIdx.x < NR * NR && a <= b && b < nel) {
+            double tr = 0.0, ti = 0.0;
+            for (int w = 0; w < warps; ++w)
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    tr += part[w][0][(g * NR + a) * 8 + g * NR + b];
+                    ti += part[w][1][(g * NR + a) * 8 + g * NR + b];
+                }
+            if (a == b) {
+                diag[a] = tr;
+                if (isfinite(ti)) ti = 0.0;                  /* |y|^2 has no imaginary part */
+            }
+            if (w1 && m > 0) {
+                float2 *Rk = R + (long long)k * nel * nel;
+                float2 v = Rk[a * nel + b];
+                Rk[a * nel + b] = make_float2((float)((double)v.x + tr), (float)((double)v.y + ti));
+                if (a != b) {
+                    v = Rk[b * nel + a];
+                    Rk[b * nel + a] = make_float2((float)((double)v.x + tr), (float)((double)v.y - ti));
+                }
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (w1) counts[k] += (uint32_t)m;
+            if (w2) {
+                const double inv = m ? 1.0 / (double)m : 0.0;
+                double across = 0.0;
+                for (int e = 0; e < nel; ++e) {
+                    if (pwr) pwr[(long long)e * nchan + k] = (float)(diag[e] * inv);
+                    across += diag[e] * inv;
+                }
+                if (mean_pwr) mean_pwr[k] = (float)(across / (double)nel);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+/* warps per channel: 4 once the channels fill the chip (1024 channels: 7 CTAs
+ * an SM), more for fewer channels while a warp keeps 256 hops */
+template <int NR>
+int w12_mma(const void *out, unsigned nel, unsigned nchan, size_t m, const uint8_t *gate, void *R,
+            uint32_t *counts, float *pwr, float *mean_pwr, cudaStream_t s) {
+    const int grid = (int)(nchan < 4096 ? nchan : 4096);
+    int warps = 4;
+    if (nchan <= 512 && m >= 8 * 256) warps = 8;
+    w12_mma_kernel<NR><<<grid, 32 * warps, 0, s>>>((const float2 *)out, (int)nel, (int)nchan, (long long)m, gate,
+                                                   (float2 *)R, counts, pwr, mean_pwr);
+    return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;
+}
+
 template <int TB>
 int w12_launch(const void *out, unsigned nel, unsigned nchan, size_t m, const uint8_t *gate, void *R,
                uint32_t *counts, float *pwr, float *mean_pwr, cudaStream_t s) {
@@ -250,7 +367,7 @@ int w12_launch(const void *out, unsigned nel, unsigned nchan, size_t m, const ui
     const size_t red = (size_t)W_NT * TB * TB * 2 * sizeof(double);
     const size_t rows = ((nel + TB - 1) / TB) * TB;
     const size_t smem = red + 2 * rows * CHUNK * sizeof(float2);
-    /* TB 1 and 2 serve one and two elements (atkb_w12), TB 4 up to MAX_NEL */
+    /* TB 1 serves one element (atkb_w12), TB 4 nine to MAX_NEL */
     constexpr size_t rows_max = TB == 4 ? MAX_NEL : TB;
     constexpr size_t smem_max = (size_t)W_NT * TB * TB * 2 * sizeof(double) + 2 * rows_max * CHUNK * sizeof(float2);
     static_assert(smem_max <= 227 * 1024, "one CTA's shared memory fits an SM");
@@ -283,7 +400,9 @@ extern "C" int atkb_w12(const void *out, unsigned nel, unsigned nchan, size_t m,
         return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;
     }
     if (nel == 1) return w12_launch<1>(out, nel, nchan, m, gate, R, counts, pwr, mean_pwr, s);
-    if (nel == 2) return w12_launch<2>(out, nel, nchan, m, gate, R, counts, pwr, mean_pwr, s);
+    if (nel == 2) return w12_mma<2>(out, nel, nchan, m, gate, R, counts, pwr, mean_pwr, s);
+    if (nel <= 4) return w12_mma<4>(out, nel, nchan, m, gate, R, counts, pwr, mean_pwr, s);
+    if (nel <= 8) return w12_mma<8>(out, nel, nchan, m, gate, R, counts, pwr, mean_pwr, s);
     return w12_launch<4>(out, nel, nchan, m, gate, R, counts, pwr, mean_pwr, s);
 }
 
