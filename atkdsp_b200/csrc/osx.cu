@@ -43,44 +43,87 @@ namespace {
 
 using namespace atkb_fft;
 
-/* one run of the fold: n terms from bin address xa / x and filter h, stride
- * M bins (M = 1 << LOGM, or the runtime m when LOGM < 0) */
-template <int LOGM, bool SM>
-__device__ __forceinline__ void fold_run(float &ar, float &ai, unsigned xa, const float2 *x, const float2 *h, int n,
-                                         int m) {
-    constexpr int kUnroll = OSX_FOLD_UNROLL;
-    constexpr int XB = SM ? 8 * OSX_G : 8;      /* bytes per bin */
-    const int M = LOGM >= 0 ? (1 << (LOGM < 0 ? 0 : LOGM)) : m;
-#pragma unroll kUnroll
-    for (int j = 0; j < n; ++j) {
-        float2 xv;
-        if (SM) asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(xv.x), "=f"(xv.y) : "r"(xa + j * M * XB));
-        else xv = __ldg(x + j * M);
-        const float2 hv = __ldg(h + j * M);
-        ar = __fadd_rn(ar, __fsub_rn(__fmul_rn(xv.x, hv.x), __fmul_rn(xv.y, hv.y)));
-        ai = __fadd_rn(ai, __fadd_rn(__fmul_rn(xv.x, hv.y), __fmul_rn(xv.y, hv.x)));
-    }
+__device__ __forceinline__ void fold_add(float &ar, float &ai, float2 xv, float2 hv) {
+    ar = __fadd_rn(ar, __fsub_rn(__fmul_rn(xv.x, hv.x), __fmul_rn(xv.y, hv.y)));
+    ai = __fadd_rn(ai, __fadd_rn(__fmul_rn(xv.x, hv.y), __fmul_rn(xv.y, hv.x)));
+}
+__device__ __forceinline__ float2 lds8(unsigned a) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+    return v;
 }
 
 /* bin k of a channel's decimating fold of one spectrum (float, j ascending,
- * the reference's rounded expression, src/channelizer.c:707-716). The bins
- * k + j*M + shift run up to nfft and then wrap once: two runs of a fixed
- * stride (M a template parameter for M <= 4096, so the unrolled loads carry
- * it in their immediate offsets). SM: the spectrum is the fused kernel's
- * shared one, bin b of this block at shared address xs + b * 8 * OSX_G;
- * else global, bin b at X[b]. */
-template <int LOGM, bool SM>
-__device__ __forceinline__ double2 fold_bin(const float2 *X, unsigned xs, const float2 *__restrict__ H, int k,
-                                            int m, int decim, int shift, int nfft) {
-    constexpr int XB = SM ? 8 * OSX_G : 8;
+ * the reference's rounded expression, src/channelizer.c:707-716): the bins
+ * k + j*M + shift, which run up to nfft (a power of two) and wrap once.
+ * The fused kernel's spectrum, bin b of this block at shared address
+ * xs + b * 8 * OSX_G. The filter does not wrap, so its values come in batches
+ * a batch ahead: with the batch's own loads only, a batch waited for L2 (the
+ * channels' filters are larger than the L1 that the spectra leave): 90 to 108
+ * cycles a term a warp with 16 warps, now 80 to 85, where the shared and L1
+ * load path is the bound. 64 channels of nfft 4096, 512 blocks: the group
+ * kernel cold 235 -> 180 us (four of a batch in flight are slower than eight,
+ * sixteen spill). */
+template <int LOGM>
+__device__ __forceinline__ double2 fold_shared(unsigned xs, const float2 *__restrict__ H, int k, int decim, int shift,
+                                               int nfft) {
+    constexpr int M = 1 << LOGM, U = OSX_FOLD_UNROLL;
+    constexpr unsigned XB = 8 * OSX_G;
+    const unsigned mask = (unsigned)nfft * XB - 1;               /* bytes of the spectrum */
+    unsigned at = ((unsigned)(k + shift) * XB) & mask;
+    const float2 *h = H + k;
+    float ar = 0.0f, ai = 0.0f;
+    int j = 0;
+    if (decim >= U) {                                            /* then a multiple of U */
+        float2 next[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) next[u] = __ldg(h + u * M);
+        for (; j < decim; j += U) {
+            float2 hv[U], xv[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) hv[u] = next[u];
+            h += U * M;
+            if (j + U < decim) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) next[u] = __ldg(h + u * M);
+            }
+            if (at + (unsigned)((U - 1) * M) * XB <= mask) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) xv[u] = lds8(xs + at + (unsigned)(u * M) * XB);
+            } else {
+#pragma unroll
+                for (int u = 0; u < U; ++u) xv[u] = lds8(xs + ((at + (unsigned)(u * M) * XB) & mask));
+            }
+            at = (at + (unsigned)(U * M) * XB) & mask;
+#pragma unroll
+            for (int u = 0; u < U; ++u) fold_add(ar, ai, xv[u], hv[u]);
+        }
+    } else {
+        for (; j < decim; ++j) fold_add(ar, ai, lds8(xs + ((at + (unsigned)(j * M) * XB) & mask)), __ldg(h + j * M));
+    }
+    return make_double2((double)ar, (double)ai);
+}
+
+/* the same from a spectrum in global memory, bin b at X[b]: two runs of a
+ * fixed stride (M a template parameter for M <= 4096, so the unrolled loads
+ * carry it in their immediate offsets; else m with LOGM < 0) */
+template <int LOGM>
+__device__ __forceinline__ void fold_run(float &ar, float &ai, const float2 *x, const float2 *h, int n, int m) {
+    const int M = LOGM >= 0 ? (1 << (LOGM < 0 ? 0 : LOGM)) : m;
+#pragma unroll 8
+    for (int j = 0; j < n; ++j) fold_add(ar, ai, __ldg(x + j * M), __ldg(h + j * M));
+}
+template <int LOGM>
+__device__ __forceinline__ double2 fold_bin(const float2 *X, const float2 *__restrict__ H, int k, int m, int decim,
+                                            int shift, int nfft) {
     const int M = LOGM >= 0 ? (1 << (LOGM < 0 ? 0 : LOGM)) : m;
     float ar = 0.0f, ai = 0.0f;
     int start = k + shift;
     if (start >= nfft) start -= nfft;
     const int jw = min(decim, (nfft - start + M - 1) / M);        /* start + j*M < nfft */
-    fold_run<LOGM, SM>(ar, ai, xs + start * XB, X + start, H + k, jw, m);
+    fold_run<LOGM>(ar, ai, X + start, H + k, jw, m);
     const int s2 = start + jw * M - nfft;
-    fold_run<LOGM, SM>(ar, ai, xs + s2 * XB, X + s2, H + k + jw * M, decim - jw, m);
+    fold_run<LOGM>(ar, ai, X + s2, H + k + jw * M, decim - jw, m);
     return make_double2((double)ar, (double)ai);
 }
 
@@ -88,12 +131,17 @@ template <bool SM>
 __device__ __forceinline__ double2 fold_any(int logm, const float2 *X, unsigned xs, const float2 *H, int k, int decim,
                                             int shift, int nfft) {
     switch (logm) {
-#define OSX_FOLD_CASE(L) case L: return fold_bin<L, SM>(X, xs, H, k, 1 << L, decim, shift, nfft);
+#define OSX_FOLD_CASE(L)                                                                       \
+    case L:                                                                                    \
+        if constexpr (SM) return fold_shared<L>(xs, H, k, decim, shift, nfft);                 \
+        else return fold_bin<L>(X, H, k, 1 << L, decim, shift, nfft);
         OSX_FOLD_CASE(1) OSX_FOLD_CASE(2) OSX_FOLD_CASE(3) OSX_FOLD_CASE(4) OSX_FOLD_CASE(5)
         OSX_FOLD_CASE(6) OSX_FOLD_CASE(7) OSX_FOLD_CASE(8) OSX_FOLD_CASE(9) OSX_FOLD_CASE(10)
         OSX_FOLD_CASE(11) OSX_FOLD_CASE(12)
 #undef OSX_FOLD_CASE
-    default: return fold_bin<-1, SM>(X, xs, H, k, 1 << logm, decim, shift, nfft);   /* M > 4096 */
+    default:                                                    /* M > 4096: never of a shared spectrum */
+        if constexpr (SM) return make_double2(0.0, 0.0);
+        else return fold_bin<-1>(X, H, k, 1 << logm, decim, shift, nfft);
     }
 }
 
@@ -353,13 +401,28 @@ __global__ void __launch_bounds__(128) osx_resample_batch_kernel(const __grid_co
     const float mu = __double2float_rn(__dsub_rn(ph, (double)b));
     const float *pp = D.pd, *dd = D.pd + (size_t)P * Q;
     float ar = 0.0f, ai = 0.0f;
-    for (int q = 0; q < Q; ++q) {
-        const long long mm = i - q;
-        if (mm < -(long long)Q) break;                          /* older than the kept history */
-        const float2 xv = __ldg(x + mm);
-        const float c = __fadd_rn(__ldg(pp + b + q * P), __fmul_rn(mu, __ldg(dd + b + q * P)));
-        ar = __fadd_rn(ar, __fmul_rn(c, xv.x));
-        ai = __fadd_rn(ai, __fmul_rn(c, xv.y));
+    /* the taps that reach no further back than the kept history, eight taps'
+     * loads in flight (with the test in the loop each tap waited for its
+     * own loads: 32 channels' 48,000 outputs 70 us cold, now 23) */
+    const long long reach = i + Q + 1;
+    const int nq = reach < Q ? (reach < 0 ? 0 : (int)reach) : Q;
+    for (int q0 = 0; q0 < nq; q0 += 8) {
+        float2 xv[8];
+        float p0[8], d0[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (q0 + u < nq) {
+                xv[u] = __ldg(x + (i - q0 - u));
+                p0[u] = __ldg(pp + b + (q0 + u) * P);
+                d0[u] = __ldg(dd + b + (q0 + u) * P);
+            }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (q0 + u < nq) {
+                const float c = __fadd_rn(p0[u], __fmul_rn(mu, d0[u]));
+                ar = __fadd_rn(ar, __fmul_rn(c, xv[u].x));
+                ai = __fadd_rn(ai, __fmul_rn(c, xv[u].y));
+            }
     }
     float2 *o = D.outs ? (float2 *)D.outs[e] + D.out_off : (float2 *)D.stage + (long long)e * D.stage_stride;
     o[k] = make_float2(ar, ai);
