@@ -1576,7 +1576,6 @@ struct atkdsp_gpu_batch {
     int *d_counters;
     int grid, smem;
     void *tk[2];                  /* timing events around the tile kernel */
-    int generic_smem;             /* the generic banks' shared memory, 0: none */
     const atkb_bank *bank;        /* the one bank of every handle, or NULL */
 };
 
@@ -1612,9 +1611,7 @@ ATKDSP_API atkdsp_gpu_batch *atkdsp_gpu_batch_create(atkdsp_pfb *const *handles,
     if (!b->h) { free(b); return NULL; }
     for (i = 0; i < count; ++i) {
         b->h[i] = handles[i];
-        /* generic banks' tiles run in a launch of their own */
-        int *most = handles[i]->bank.plan.fast ? &b->smem : &b->generic_smem;
-        if (handles[i]->bank.smem_bytes > *most) *most = handles[i]->bank.smem_bytes;
+        if (handles[i]->bank.smem_bytes > b->smem) b->smem = handles[i]->bank.smem_bytes;
     }
     for (i = 1; i < count && handles[i]->be == handles[0]->be; ++i) {}
     if (i == count) b->bank = &handles[0]->be->bank;
@@ -1663,9 +1660,6 @@ ATKDSP_API float atkdsp_gpu_batch_kernel_ms(atkdsp_gpu_batch *b) {
 static int batch_enqueue(atkdsp_gpu_batch *b, int slot, void *stream) {
     int rc = atkb_h2d(b->d_tables, b->h_tables[slot], b->tbl_bytes, stream);
     if (rc == ATKB_OK) rc = atkb_event_record_node(b->tk[0], stream);
-    if (rc == ATKB_OK && b->generic_smem)
-        rc = atkb_pfb_generic_tiles(tbl_jobs(b->d_tables), tbl_tiles(b->d_tables, b->count), (int)b->count,
-                                    b->d_counters, b->generic_smem, stream);
     if (rc == ATKB_OK)
         rc = atkb_pfb_launch(tbl_jobs(b->d_tables), tbl_tiles(b->d_tables, b->count),
                              tbl_carry(b->d_tables, b->count), (int)b->count, b->d_counters, b->grid,

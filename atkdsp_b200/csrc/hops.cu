@@ -260,29 +260,6 @@ pfb_generic1_kernel(const __grid_constant__ atkb_job J, const __grid_constant__ 
     else generic_cta<NTH>(J, cre, cim, (long long)blockIdx.x * gh, gh, SB, counters);
 }
 
-/* the generic banks' tiles of a batch (tables as the tile kernel's, which
- * passes them over and copies the carries): a fixed grid over all tiles, each
- * CTA taking every gridDim-th, so that it can be captured once */
-__global__ void __launch_bounds__(256, 4)
-pfb_generic_tiles_kernel(const atkb_job *__restrict__ jobs, const int *__restrict__ tile_start, int njobs,
-                         int *counters) {
-    __shared__ atkb_bank SB;
-    const int total = tile_start[njobs];
-    for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
-        int lo = 0, hi = njobs - 1;             /* the last job whose first tile <= tile */
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (tile_start[mid] <= tile) lo = mid;
-            else hi = mid - 1;
-        }
-        const atkb_bank *B = jobs[lo].bank;
-        if (B->plan.fast || B->plan.big) continue;
-        __syncthreads();                        /* the last tile's reads of SB and of the points */
-        generic_cta<256>(jobs[lo], jobs[lo].cre, jobs[lo].cim, (long long)(tile - tile_start[lo]) * B->tile_hops,
-                         B->tile_hops, SB, counters);
-    }
-}
-
 }  // namespace
 
 /* threads of a hop's CTA: two branches each, 64 to 512 */
@@ -351,25 +328,6 @@ static int generic_launch(const atkb_job *jobs, const atkb_carry *carries, bool 
     const size_t smem = (size_t)nchan * gh * 32;
     if (one) pfb_generic1_kernel<NTH><<<(unsigned)grid, NTH, smem, st>>>(*jobs, *carries, groups, gh, d_counters);
     else pfb_generic_kernel<NTH><<<(unsigned)grid, NTH, smem, st>>>(jobs, carries, njobs, groups, gh, d_counters);
-    return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;
-}
-
-extern "C" int atkb_pfb_generic_tiles(const atkb_job *d_jobs, const int *d_tile_start, int njobs, int *d_counters,
-                                      int smem_bytes, void *stream) {
-    static std::atomic<bool> configured[64];
-    int dev = 0, per_sm = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return ATKB_E_NODEV;
-    if (!configured[dev].load(std::memory_order_acquire)) {
-        if (cudaFuncSetAttribute(pfb_generic_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 6400 * 32) !=
-            cudaSuccess)
-            return ATKB_E_KERNEL;
-        configured[dev].store(true, std::memory_order_release);
-    }
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pfb_generic_tiles_kernel, 256, smem_bytes) !=
-        cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    pfb_generic_tiles_kernel<<<per_sm * atkb_sm_count(dev), 256, smem_bytes, (cudaStream_t)stream>>>(
-        d_jobs, d_tile_start, njobs, d_counters);
     return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;
 }
 

@@ -243,10 +243,6 @@ int  atkb_pfb_hops_ok(const atkb_bank *B);
  * job and its carry in host memory, passed as launch parameters */
 int  atkb_pfb_generic(const atkb_job *jobs, const atkb_carry *carries, int one, int njobs, int m, int nchan,
                       int *d_counters, void *stream);
-/* the tiles of a batch whose banks are generic (the tile kernel passes them
- * over), smem_bytes the largest of their banks'; launched beside it */
-int  atkb_pfb_generic_tiles(const atkb_job *d_jobs, const int *d_tile_start, int njobs, int *d_counters,
-                            int smem_bytes, void *stream);
 /* the int16 constants of nel device jobs and carries whose doff is set, from
  * that device-held offset (after the table upload, before the tile kernel) */
 int  atkb_pfb_conv_from_offset(atkb_job *d_jobs, atkb_carry *d_carry, int nel, void *stream);

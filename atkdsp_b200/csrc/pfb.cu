@@ -34,13 +34,25 @@
  *     load per butterfly, group barriers), the last pass fused with the
  *     rotation, cal, rounding and the transpose to channel-major; each
  *     channel gets a run of tile_hops consecutive outputs.
- *   - Any other M up to 6400 has kernels of its own (hops.cu): here its tiles
- *     are passed over and its carries copied.
+ *   - Any other M up to 6400: single handles have kernels of their own
+ *     (hops.cu); a batch's tiles run the same passes here (pfb_generic.cuh).
  */
 #include <atomic>
 #include "pfb_kernel.cuh"
 
 namespace {
+
+#include "pfb_generic.cuh"
+
+/* a generic bank's tile in a batch: the passes of the single handles' kernel,
+ * out of line so that its registers are its own. (A launch of its own before
+ * the tile kernel ran the six-scale bank, 8 to 256 channels in chunks of
+ * 65,536 samples, at 769 MS/s; inside, where the tiles of all scales overlap,
+ * at 1,238.) */
+__device__ __noinline__ void tile_generic(const atkb_job &J, const atkb_bank &B, long long h0, int nvalid,
+                                          double2 *sm) {
+    generic_tile<NT>(J, B, J.cre, J.cim, h0, nvalid, sm);
+}
 
 struct AllShapes {
     static __device__ __forceinline__ void run(int key, const atkb_job &J, const atkb_bank &SB, long long h0,
@@ -52,7 +64,8 @@ struct AllShapes {
         T(12) T(16 + 12) T(32 + 12) T(48 + 12) EACH(80) EACH(96)
 #undef T
 #undef EACH
-        default: break;
+        case -1: break;                      /* a tile to skip */
+        default: tile_generic(J, SB, h0, nvalid, sm); break;
         }
     }
 };

@@ -993,8 +993,7 @@ __device__ __forceinline__ void fetch_tile(const atkb_job *__restrict__ jobs, co
     if (lane == 0) s_local[slot] = tile - tile_start[lo];
 }
 
-/* RUN::run(key, ...) does one tile, or nothing for a key it does not know (a
- * generic bank's tile, which pfb_generic_tiles_kernel has, or one to skip) */
+/* RUN::run(key, ...) does one tile, or nothing for key -1, a tile to skip */
 template <class RUN>
 __device__ __forceinline__ void tiles_loop(const atkb_job *__restrict__ jobs, const int *__restrict__ tile_start,
                                            const atkb_carry *__restrict__ carries, int njobs,

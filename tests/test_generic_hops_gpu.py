@@ -1,5 +1,5 @@
 """Filterbanks whose nchan is no power of two (or below 16): single handles run
-a kernel of one CTA per few hops, batches one over their tiles, both through
+a kernel of one CTA per few hops, batches the tile kernel, both through
 the same mixed-radix passes (butterflies for 2, 3, 4, 5, 7, 8, a direct DFT for
 other primes). Every radix, hop counts that leave a CTA's last group short,
 one and two elements, cf32 and int16: device calls against a batch bit for bit
