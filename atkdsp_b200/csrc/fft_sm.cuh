@@ -148,59 +148,34 @@ __device__ __forceinline__ void dft8(double2 *v, bool inv) {
     v[7] = d2sub(e[3], t3);
 }
 
-/* ---- butterflies with their twiddles in the multiply-adds --------------------
- * R = 2^L points as L levels of radix-2 butterflies a, b -> a + w b, a - w b,
- * six fused multiply-adds each (the second output is 2a minus the first); the
- * input twiddles W^(r k) and the constant roots fold into each level's w, all
- * from the one table entry w = W^k: 10.5 double operations a point at radix 8
- * with the twiddles, where separate products and a split DFT take 13. X[k] is
- * left at v[brev(k)]. Forward transforms only. */
-__device__ __forceinline__ void bfly2(double2 &a, double2 &b, double2 w) {
-    const double tx = __fma_rn(-w.y, b.y, __fma_rn(w.x, b.x, a.x));
-    const double ty = __fma_rn(w.y, b.x, __fma_rn(w.x, b.y, a.y));
-    b = make_double2(__fma_rn(2.0, a.x, -tx), __fma_rn(2.0, a.y, -ty));
-    a = make_double2(tx, ty);
-}
-/* the same with -i w */
-__device__ __forceinline__ void bfly2_mi(double2 &a, double2 &b, double2 w) {
-    bfly2(a, b, make_double2(w.y, -w.x));
-}
-__device__ __forceinline__ double2 mul_w8(double2 w) {
-    const double h = 0.70710678118654752440;
-    return make_double2(h * (w.x + w.y), h * (w.y - w.x));
-}
+/* the forward radix-R butterfly of a later pass, the operations and order of
+ * fft_r8's passes: every leg but the first multiplied once by its twiddle
+ * W^(r k), then the plain DFT. w: the table entry of W^k. */
 template <int R>
-__device__ __forceinline__ void dft_tw(double2 *v, double2 w) {
-    if constexpr (R == 2) {
-        bfly2(v[0], v[1], w);
+__device__ __forceinline__ void dft_tw(double2 *v, const double2 *__restrict__ w, int k, int sh) {
+    const double2 w1 = __ldg(w + (k << sh));
+    if constexpr (R == 8) {
+        const double2 w2 = d2sq(w1), w3 = d2mul(w2, w1), w4 = d2sq(w2);
+        v[1] = d2mul(v[1], w1);
+        v[2] = d2mul(v[2], w2);
+        v[3] = d2mul(v[3], w3);
+        v[4] = d2mul(v[4], w4);
+        v[5] = d2mul(v[5], d2mul(w4, w1));
+        v[6] = d2mul(v[6], d2sq(w3));
+        v[7] = d2mul(v[7], d2mul(w4, w3));
+        dft8(v, false);
+    } else if constexpr (R == 4) {
+        v[1] = d2mul(v[1], w1);
+        v[2] = d2mul(v[2], __ldg(w + (2 * k << sh)));
+        v[3] = d2mul(v[3], __ldg(w + (3 * k << sh)));
+        dft4(v, false);
     } else {
-        const double2 w2 = d2sq(w);
-        if constexpr (R == 4) {
-            bfly2(v[0], v[2], w2);
-            bfly2(v[1], v[3], w2);
-            bfly2(v[0], v[1], w);
-            bfly2_mi(v[2], v[3], w);
-        } else {
-            const double2 w4 = d2sq(w2), we = mul_w8(w);
-#pragma unroll
-            for (int r = 0; r < 4; ++r) bfly2(v[r], v[r + 4], w4);
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                bfly2(v[r], v[r + 2], w2);
-                bfly2_mi(v[4 + r], v[6 + r], w2);
-            }
-            bfly2(v[0], v[1], w);
-            bfly2_mi(v[2], v[3], w);
-            bfly2(v[4], v[5], we);
-            bfly2_mi(v[6], v[7], we);
-        }
+        const double2 c = d2mul(v[1], w1);
+        v[1] = d2sub(v[0], c);
+        v[0] = d2add(v[0], c);
     }
 }
-template <int R>
-__host__ __device__ constexpr int brev(int k) {
-    return R == 2 ? k : R == 4 ? (k & 1) * 2 + (k >> 1) : (k & 1) * 4 + (k & 2) + (k >> 2);
-}
-/* sw of swz, with which point STEP * r past the one at byte offset a (whose
+/* swz, with which point STEP * r past the one at byte offset a (whose
  * index has no bits there) is one XOR away, plus a constant above bit 5 */
 template <int STEP>
 __device__ __forceinline__ double2 &swz_at(double2 *sm, int a, int r) {

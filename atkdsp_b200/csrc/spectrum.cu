@@ -15,12 +15,14 @@
  * are exact in any order; the sums differ from a one-thread run only in their
  * rounding sequence.
  *
- * What bounds it: the double pipe (about 45 operations a point) and the three
+ * What bounds it: the double pipe (about 54 operations a point) and the three
  * shared-memory exchanges of 32 bytes a point at n 4096; HBM has a tenth of
- * the time. 2^24 samples, n 4096, hop 2048, Hann, the four statistics: 248 us
- * (67 GS/s), against 710 us with the accumulators in shared memory, the
- * samples staged there before the first pass and one thread per bin merging
- * the partial lines (480 us of frames, 328 of merging).
+ * the time. 2^24 samples, n 4096, hop 2048, Hann, the four statistics: 244 us
+ * (69 GS/s), 710 us with the accumulators in shared memory and one thread per
+ * bin merging the partial lines. A leg is multiplied by its whole twiddle once,
+ * as in fft_r8: radix-2 steps with the twiddles folded into multiply-adds (and
+ * a - w b formed as 2a minus the sum) take fewer operations, ran no faster
+ * (248 us), and turned an infinite a into NaN.
  */
 #include <cuda_runtime.h>
 #include <atomic>
@@ -44,7 +46,7 @@ __device__ __forceinline__ void frame_sync() {
 }
 
 /* the passes after the first (which left Ns = 2^LOGNS) of one frame at sm, in
- * place; the last leaves bin lt + u*n/8 + r*Ns in v[u*R + brev(r)] */
+ * place; the last leaves bin lt + u*n/8 + r*Ns in v[u*R + r] */
 template <int LOGN, int LOGNS>
 struct SpecPass {
     static constexpr int REM = LOGN - LOGNS, LR = REM >= 3 ? 3 : REM, R = 1 << LR, U = 8 / R;
@@ -55,24 +57,23 @@ struct SpecPass {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int j = lt + u * G, k = j & (NS - 1), a = swz(j) * 16;
-            const double2 w = __ldg(tw + (k << (LOGN - LOGNS - LR)));
 #pragma unroll
             for (int r = 0; r < R; ++r) v[u * R + r] = swz_at<NR>(sm, a, r);
-            dft_tw<R>(v + u * R, w);
+            dft_tw<R>(v + u * R, tw, k, LOGN - LOGNS - LR);
         }
         frame_sync<G>();                       /* every point of the frame is read */
         if constexpr (!LAST) {
             static_assert(U == 1, "a middle pass is radix 8");
             const int k = lt & (NS - 1), d = swz(((lt - k) << 3) + k) * 16;
 #pragma unroll
-            for (int r = 0; r < 8; ++r) swz_at<NS>(sm, d, r) = v[brev<8>(r)];
+            for (int r = 0; r < 8; ++r) swz_at<NS>(sm, d, r) = v[r];
             frame_sync<G>();
             Next::run(sm, v, tw, lt);
         }
     }
     /* of the last pass: where value i of v belongs */
     static __device__ __forceinline__ int bin(int i, int lt) {
-        if constexpr (LAST) return lt + (i / R) * G + brev<R>(i % R) * NS;   /* brev is its own inverse */
+        if constexpr (LAST) return lt + (i / R) * G + (i % R) * NS;
         else return Next::bin(i, lt);
     }
 };

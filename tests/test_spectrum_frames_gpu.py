@@ -57,3 +57,24 @@ def test_nan_frames(n):
             got = line.cpu().numpy()
             assert np.array_equal(np.isnan(got), np.isnan(ref)), (at, det)
             assert np.nanmax(np.abs(got - ref), initial=0.0) <= 1e-4, (at, det)
+
+
+@pytest.mark.parametrize("n", [16, 64, 256, 512, 4096])
+def test_an_infinite_sample_reaches_every_bin(n):
+    """A sample whose index is a multiple of n/8 meets only +-1, +-i and W8
+    before the additions (leg 0 of every later pass), so no 0 x infinity
+    arises: every bin of its frame is infinite, as the transform's sum is."""
+    from atkdsp_b200.gpu import Spectrum
+    rng = np.random.default_rng(n)
+    x = (rng.standard_normal(9 * n) + 1j * rng.standard_normal(9 * n)).astype(np.complex64)
+    sp = Spectrum(n)
+    for at in (0, n // 8, n // 2, 7 * n // 8):
+        y = x.copy()
+        y[4 * n + at] = np.inf
+        for det in ("max", "avg"):
+            line, _ = sp.reduce(_t(y), n, None, det)
+            assert np.all(np.isposinf(line.cpu().numpy())), (at, det)
+        line, _ = sp.reduce(_t(y), n, None, "min")
+        assert np.all(np.isfinite(line.cpu().numpy())), at
+        st = sp.stats(_t(y), n, None)
+        assert np.all(np.isposinf(st["max"].cpu().numpy())) and np.all(np.isfinite(st["min"].cpu().numpy())), at
