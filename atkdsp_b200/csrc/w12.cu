@@ -251,12 +251,12 @@ __global__ void cov_reset_kernel(float2 *R, uint32_t *counts, int nel, int nchan
  * the cross-group blocks of the product are not used. Each warp of a channel's
  * CTA takes a run of hops; the warps' sums are added in warp order.
  *
- * The tile-per-thread kernel converts every sample three times for 8
- * elements, spends a quarter of its passes on one hop in 85, and sums 85
- * partials in 48 threads; this one is bound by the matrix unit's double rate
- * (256 products a hop, 16 us) and the samples' trip from L2. Before and after,
- * us: 8 elements x 2048 channels x 513 hops 88.3, 30.2; 8 x 256 x 4097 53.5,
- * 26.9; 4 x 2048 x 513 76.1, 20.2; 2 x 1024 x 2000 23.9, 15.6. */
+ * Bound by the matrix unit's double rate (256 products a hop: 16 us of the
+ * first figure) and the samples' trip from L2. us, the tile-per-thread kernel
+ * and this one: 8 elements x 2048 channels x 513 hops 88.3, 30.2; 8 x 256 x
+ * 4097 53.5, 26.9; 4 x 2048 x 513 76.1, 20.2; 2 x 1024 x 2000 23.9, 15.6. */
+#define MMA_WARPS 16
+#define MMA_U 8          /* loads in flight a lane */
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                  : "+d"(c[0]), "+d"(c[1])
@@ -264,12 +264,12 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 }
 
 template <int NR>
-__global__ void __launch_bounds__(W_NT)
+__global__ void __launch_bounds__(32 * MMA_WARPS)
 w12_mma_kernel(const float2 *__restrict__ out, int nel, int nchan, long long m, const uint8_t *__restrict__ gate,
                float2 *__restrict__ R, uint32_t *__restrict__ counts, float *__restrict__ pwr,
                float *__restrict__ mean_pwr) {
-    constexpr int G = 8 / NR, STEP = 4 * G, U = 8;
-    __shared__ double part[W_NT / 32][2][64];
+    constexpr int G = 8 / NR, STEP = 4 * G, U = MMA_U;
+    __shared__ double part[MMA_WARPS][2][64];
     __shared__ double diag[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int row = lane >> 2, el = row % NR;
@@ -345,14 +345,20 @@ w12_mma_kernel(const float2 *__restrict__ out, int nel, int nchan, long long m, 
     }
 }
 
-/* warps per channel: 4 once the channels fill the chip (1024 channels: 7 CTAs
- * an SM), more for fewer channels while a warp keeps 256 hops */
+/* Warps per channel: the most of 16, 8 and 4 that leaves each three turns of
+ * the loop (256 / NR hops a turn). A long run is bound by the loads in flight,
+ * a short one by the reduction over the warps and, with many channels, by how
+ * many CTAs an SM holds. us at 4 / 8 / 16 warps: 8 elements x 1024 channels x
+ * 20,000 hops 902 / 651 / 358 (9 to 32 elements' kernel 727), 4 x 64 x 200,000
+ * 1085 / 557 / 304 (537), 8 x 4096 x 1000 102 / 83 / 95, 8 x 2048 x 256 19 /
+ * 20 / 35, 2 x 4096 x 256 19 / 30 / 61. */
 template <int NR>
 int w12_mma(const void *out, unsigned nel, unsigned nchan, size_t m, const uint8_t *gate, void *R,
             uint32_t *counts, float *pwr, float *mean_pwr, cudaStream_t s) {
     const int grid = (int)(nchan < 4096 ? nchan : 4096);
-    int warps = 4;
-    if (nchan <= 512 && m >= 8 * 256) warps = 8;
+    constexpr size_t turns = 3 * MMA_U * 4 * (8 / NR);
+    int warps = MMA_WARPS;
+    while (warps > 4 && m < warps * turns) warps /= 2;
     w12_mma_kernel<NR><<<grid, 32 * warps, 0, s>>>((const float2 *)out, (int)nel, (int)nchan, (long long)m, gate,
                                                    (float2 *)R, counts, pwr, mean_pwr);
     return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;

@@ -80,3 +80,27 @@ def test_infinities_and_nan_stay_in_their_entries(nel):
     bad[3, 1, :] = bad[3, :, 1] = bad[5, 0, :] = bad[5, :, 0] = True
     assert np.isfinite(got[~bad]).all() and not np.isfinite(got[bad]).any()
     assert got[3, 1, 1].real == np.inf and np.isnan(got[5, 0, 0].real)
+
+
+@pytest.mark.parametrize("nel,ms", [(2, (3071, 3072, 6143, 6145)), (3, (1535, 1536, 3073)), (4, (3071, 3072)),
+                                    (5, (767, 1537)), (8, (767, 768, 1535, 1536, 9001))])
+def test_runs_around_the_warp_counts(nel, ms):
+    """4, 8 and 16 warps a channel: hop counts around the lines between them,
+    where a warp's run is shortest and the last may be empty."""
+    from atkdsp_b200 import gpu
+    M = 5
+    for m in ms:
+        rng = np.random.default_rng(nel * 7 + m)
+        y = (rng.standard_normal((nel, M, m)) + 1j * rng.standard_normal((nel, M, m))).astype(np.complex64)
+        R = torch.zeros(M, nel, nel, dtype=torch.complex64, device="cuda")
+        c = torch.zeros(M, dtype=torch.int32, device="cuda")
+        d = torch.from_numpy(y).cuda()
+        gpu.cov_accumulate(d, nel, M, None, R, c)
+        pw, mean = gpu.channel_power(d, nel, M)
+        torch.cuda.synchronize()
+        got, re, im, mag = R.cpu().numpy(), *_sums(y)
+        assert np.array_equal(c.cpu().numpy(), np.full(M, m)), m
+        _close(got.real, re, mag, m)
+        _close(got.imag, im, mag, m)
+        want = np.diagonal(re, axis1=1, axis2=2).T / m
+        assert (np.abs(pw.cpu().numpy() - want) <= 2.0 ** -23 * want).all(), m
