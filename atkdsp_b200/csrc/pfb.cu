@@ -44,28 +44,39 @@ namespace {
 
 #include "pfb_generic.cuh"
 
-/* a generic bank's tile in a batch: the passes of the single handles' kernel,
- * out of line so that its registers are its own. (A launch of its own before
- * the tile kernel ran the six-scale bank, 8 to 256 channels in chunks of
- * 65,536 samples, at 769 MS/s; inside, where the tiles of all scales overlap,
- * at 1,238.) */
-__device__ __noinline__ void tile_generic(const atkb_job &J, const atkb_bank &B, long long h0, int nvalid,
-                                          double2 *sm) {
-    generic_tile<NT>(J, B, J.cre, J.cim, h0, nvalid, sm);
+/* Every shape's tile, and the generic banks', is a function of its own, so
+ * that each gets the 64 registers for itself: with all of them inline one
+ * allocation served 50 shapes with 1.5 to 1.9 KB of spills, and a change in
+ * any one (the generic branch above all) moved the others by up to 12 %.
+ * us, all inline / apart: 64 uneven streams 1090 / 1070, another 64 1271 /
+ * 1233, 256 of them 5293 / 5181. The generic tile loads one tap at a time:
+ * eight in flight need more registers than are left. Six scales of 8 to 256
+ * channels, chunks of 65,536 samples: 1255 / 1450 MS/s. */
+__device__ __noinline__ void tile_generic(const atkb_job &__restrict__ J, const atkb_bank &__restrict__ B,
+                                          long long h0, int nvalid) {
+    extern __shared__ double2 sm[];
+    generic_tile<NT, 1>(J, B, J.cre, J.cim, h0, nvalid, sm);
+}
+
+template <int KEY>
+__device__ __noinline__ void tile_of(const atkb_job &__restrict__ J, const atkb_bank &__restrict__ B, long long h0,
+                                     int nvalid) {
+    extern __shared__ double2 sm[];
+    run_tile<KEY>(J, B, h0, nvalid, sm, (float2 *)sm);
 }
 
 struct AllShapes {
     static __device__ __forceinline__ void run(int key, const atkb_job &J, const atkb_bank &SB, long long h0,
-                                               int nvalid, double2 *sm, float2 *to) {
+                                               int nvalid, double2 *, float2 *) {
         switch (key) {
-#define T(K) case K: run_tile<K>(J, SB, h0, nvalid, sm, to); break;
+#define T(K) case K: tile_of<K>(J, SB, h0, nvalid); break;
 #define EACH(S) T(S + 4) T(S + 5) T(S + 6) T(S + 7) T(S + 8) T(S + 9) T(S + 10)
         EACH(0) T(11) EACH(16) EACH(32) EACH(48) T(16 + 11) T(32 + 11) T(48 + 11)
         T(12) T(16 + 12) T(32 + 12) T(48 + 12) EACH(80) EACH(96)
 #undef T
 #undef EACH
         case -1: break;                      /* a tile to skip */
-        default: tile_generic(J, SB, h0, nvalid, sm); break;
+        default: tile_generic(J, SB, h0, nvalid); break;
         }
     }
 };

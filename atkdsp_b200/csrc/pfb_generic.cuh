@@ -108,7 +108,7 @@ __device__ __noinline__ void direct_pass(const double2 *__restrict__ src, double
 
 /* hops h0 .. h0 + nvalid of job J (int16 constants cre, cim) through `sm`
  * (2 * nvalid * nchan points) by NTH threads */
-template <int NTH>
+template <int NTH, int U = 8>
 __device__ __forceinline__ void generic_tile(const atkb_job &J, const atkb_bank &B, float cre, float cim, long long h0,
                                           int nvalid, double2 *sm) {
     const int M = B.nchan, K = B.K;
@@ -119,17 +119,17 @@ __device__ __forceinline__ void generic_tile(const atkb_job &J, const atkb_bank 
         const unsigned tt = e / (unsigned)M, q = e - tt * M;
         const long long base = (h0 + tt) * (long long)B.hop + q;
         float fr = -0.0f, fi = -0.0f;
-        for (int k0 = 0; k0 < K; k0 += 8) {            /* eight taps' loads in flight */
-            float h[8];
-            float2 x[8];
+        for (int k0 = 0; k0 < K; k0 += U) {            /* U taps' loads in flight */
+            float h[U];
+            float2 x[U];
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
+            for (int u = 0; u < U; ++u)
                 if (k0 + u < K) {
                     h[u] = __ldg(taps + (k0 + u) * M + q);
                     x[u] = src.at(base + (k0 + u) * M);
                 }
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
+            for (int u = 0; u < U; ++u)
                 if (k0 + u < K) {
                     fr = __fadd_rn(fr, __fmul_rn(h[u], x[u].x));
                     fi = __fadd_rn(fi, __fmul_rn(h[u], x[u].y));
