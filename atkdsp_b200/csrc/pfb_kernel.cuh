@@ -406,6 +406,21 @@ struct PairStaged {                    /* the padded shared-memory window */
     }
 };
 
+/* Taps a turn of the paired fold's loop; 0 leaves it to the compiler, which in
+ * the kernels of one shape (pfb_one.cu) chose worse for a few than it had in
+ * the kernel of every shape: us there / left to it / as here, 3,000,001
+ * samples, nchan 4096 4x 12 taps 187 / 192 / 178, 4096 4x 16 199 / 205 / 193,
+ * 2048 1x 16 50.7 / 53.6 / 51.7, 16 4x 16 142 / 148 / 137, 16 2x 5 66 / 71 / 64.
+ * nchan 4096 1x is best at four (10,000,001 samples, 12 taps: 165 / 167 / 165,
+ * one tap 167). */
+__host__ __device__ constexpr int fold_unroll(int logm, int logos) {
+#ifdef ONE_LOGM
+    return logm == 4 ? 2 : logm == 12 ? (logos == 0 ? 4 : 1) : logm == 11 && logos == 0 ? 1 : 0;
+#else
+    return 0;
+#endif
+}
+
 template <int LOGM, int LOGOS, class LD>
 __device__ __forceinline__ void fold_pair(float2 (&a)[4], float2 (&b)[4], const float4 *tq, int K,
                                           bool tb_ok, const LD &ld) {
@@ -426,7 +441,7 @@ __device__ __forceinline__ void fold_pair(float2 (&a)[4], float2 (&b)[4], const 
             if (i >= D2) mac(b[i - D2], h[i - D2], x);
         }
     }
-    for (int k = 1; k < K; ++k) {
+    auto step = [&](int k) {
         const float4 cv = __ldg(tq + k * 2 * MP);
         const float h[4] = {cv.x, cv.y, cv.z, cv.w};
         const float g[4] = {pv.x, pv.y, pv.z, pv.w};
@@ -438,6 +453,13 @@ __device__ __forceinline__ void fold_pair(float2 (&a)[4], float2 (&b)[4], const 
             else mac(b[i - D2 + 4], g[i - D2 + 4], x);
         }
         pv = cv;
+    };
+    constexpr int U = fold_unroll(LOGM, LOGOS);
+    if constexpr (U == 0) {
+        for (int k = 1; k < K; ++k) step(k);
+    } else {
+#pragma unroll U
+        for (int k = 1; k < K; ++k) step(k);
     }
     if (tb_ok) {                       /* the slots past hop ta's window */
         const float g[4] = {pv.x, pv.y, pv.z, pv.w};
