@@ -26,12 +26,15 @@ atkdsp_pfb *atkb_pfb_create_served(double fs, unsigned nchan, unsigned oversampl
 /* a device call of one element and at most this many output points (hops x
  * nchan) runs one CTA per hop too. Measured per call, tile kernel / per-hop
  * kernel: nchan 1024, 2x, 16 taps 18.5 / 12.4 us at 128 hops and 20.2 / 22.5 at
- * 256; nchan 256, 2x, 8 taps 14.4 / 9.7 at 512 hops and 14.4 / 16.5 at 1024;
- * nchan 64, 2x, 16 taps 15.5 / 12.4 at 2048: the line lies at one wave of
- * 2^17 points whatever the nchan; below nchan 64 at 2048 hops, where the CTAs
- * themselves count (nchan 16, 2x, 12 taps, 8192 hops: 33 us, tile kernel 15). */
+ * 256; nchan 256, 2x, 8 taps 14.4 / 9.7 at 512 hops and 14.4 / 16.5 at 1024. */
 #define ATKB_HOPS1_POINTS ((size_t)1 << 17)
-#define ATKB_HOPS1_MAX 2048
+/* ... and at most this many hops: small filterbanks, where the CTAs count
+ * themselves (nchan 16, 2x, 12 taps, 8192 hops: 33 us, tile kernel 15), and
+ * long prototypes, whose taps and samples each hop reads for itself. 2048 hops:
+ * nchan 64, 2x, 16 taps 15.5 / 12.4, nchan 32, 1x, 20 taps 14.8 / 14.5, 32 taps
+ * 16.6 / 18.5, 128 taps 44 / 44 (2x: 30 / 43); 1536 hops: 32 taps faster at
+ * nchan 16 to 64; 1024 hops: nchan 16, 1x, 128 taps 29 / 24, nchan 128 44 / 43. */
+static inline size_t atkb_hops1_max(unsigned taps) { return taps <= 20 ? 2048 : taps <= 32 ? 1536 : 1024; }
 /* ... and write at most this many outputs straight into pinned host memory */
 #define ATKB_DIRECT_OUT 2048
 

@@ -44,3 +44,26 @@ def test_device_calls_equal_the_tile_kernel(M, os_, K, fmt):
             assert np.array_equal(y.cpu().numpy().reshape(-1).view(np.uint32),
                                   out[:M * hops].cpu().numpy().view(np.uint32)), (m, n)
         assert ak.load().atkdsp_gpu_pfb_faults(a.handle) == 0
+
+
+@pytest.mark.parametrize("M,os_,K,line", [(16, 2, 21, 1536), (32, 1, 32, 1536), (32, 2, 33, 1024), (16, 1, 40, 1024)])
+def test_long_prototypes_around_their_line(M, os_, K, line):
+    """More taps a branch move the line to fewer hops; on both sides of it the
+    outputs and the carried state are the tile kernel's."""
+    from atkdsp_b200 import gpu
+    rng = np.random.default_rng(M + K)
+    hop = M // os_
+    for m in (line, line + 1):
+        a, b = ak.Pfb(FS, M, os_, K), ak.Pfb(FS, M, os_, K)
+        batch = gpu.Batch([b])
+        for n in (m * hop, 5 * hop + 1):
+            x = torch.from_numpy((rng.standard_normal(n) + 1j * rng.standard_normal(n)).astype(np.complex64)).cuda()
+            y = gpu.process_n(a, [x], 1)
+            hops = b.out_hops(n)
+            out = torch.zeros(max(M * hops, 1), dtype=torch.complex64, device="cuda")
+            torch.cuda.synchronize()
+            batch.process([x], [out])
+            torch.cuda.synchronize()
+            assert np.array_equal(y.cpu().numpy().reshape(-1).view(np.uint32),
+                                  out[:M * hops].cpu().numpy().view(np.uint32)), (m, n)
+        assert ak.load().atkdsp_gpu_pfb_faults(a.handle) == 0
