@@ -45,7 +45,8 @@ __device__ __forceinline__ void hop_pass(const double2 *__restrict__ src, double
         dftR<R>(v);
         const int d = (j - k) * R + k;
 #pragma unroll
-        for (int r = 0; r < R; ++r) dst[d + r * Ns] = v[r];
+        for (int r = 0; r < R; ++r)
+            if (IDX_OK(d + r * Ns < M)) dst[d + r * Ns] = v[r];
     }
 }
 
@@ -73,7 +74,8 @@ __device__ __forceinline__ void hop_pass_last(const double2 *__restrict__ src, i
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int kb = j + r * Ns;
-            out[(long long)kb * J.ldo + J.out_col + t] = finish_bin(v[r], kb, s, M, osm + 1, B.hop, true, twd, cal);
+            if (IDX_OK(kb < M && J.out_col + t < J.ldo))
+                out[(long long)kb * J.ldo + J.out_col + t] = finish_bin(v[r], kb, s, M, osm + 1, B.hop, true, twd, cal);
         }
     }
 }
@@ -130,7 +132,7 @@ __device__ __forceinline__ void hop_run(const atkb_job &J, float cre, float cim,
                 float2 x[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u)
-                    if (k0 + u < K) {
+                    if (k0 + u < K && IDX_OK(base + (long long)(k0 + u) * M + q < J.nsrc)) {
                         h[u] = __ldg(taps + (long long)(k0 + u) * M + q);
                         x[u] = src.at(base + (long long)(k0 + u) * M + q);
                     }
@@ -339,6 +341,14 @@ extern "C" int atkb_pfb_generic(const atkb_job *jobs, const atkb_carry *carries,
                                  : generic_launch<512>(jobs, carries, one != 0, njobs, m, nchan, d_counters, (cudaStream_t)stream);
     atkb_range_pop();
     return rc;
+}
+
+extern "C" unsigned atkb_pfb_hops_fault(void) {
+#ifdef ATKB_DEBUG_BOUNDS
+    return take_debug_fault();
+#else
+    return 0;
+#endif
 }
 
 extern "C" int atkb_pfb_hops_ok(const atkb_bank *B) {

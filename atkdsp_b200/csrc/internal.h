@@ -216,6 +216,7 @@ int  atkb_pfb_launch_pdl(const atkb_job *d_jobs, const int *d_tile_start, const 
 /* the tile kernel of one tile key alone (pfb_one.cu), or NULL */
 const void *atkb_pfb_one(int key);
 unsigned atkb_pfb_one_fault(void);
+unsigned atkb_pfb_hops_fault(void);
 int  atkb_event_query(void *ev);        /* ATKB_OK when complete, 1 when pending */
 int  atkb_event_spin(void *ev);         /* wait for an event by polling it */
 /* large filterbanks (plan.big: nchan beyond one CTA's shared memory): hops

@@ -349,7 +349,7 @@ extern "C" int atkb_pfb_conv_from_offset(atkb_job *d_jobs, atkb_carry *d_carry, 
 
 extern "C" unsigned atkb_pfb_debug_fault(void) {
 #ifdef ATKB_DEBUG_BOUNDS
-    return take_debug_fault() | atkb_pfb_one_fault();
+    return take_debug_fault() | atkb_pfb_one_fault() | atkb_pfb_hops_fault();
 #else
     return 0;
 #endif

@@ -5,6 +5,27 @@
 #ifndef ATKB_PFB_DEV_CUH
 #define ATKB_PFB_DEV_CUH
 
+/* Per-thread index checks of the debug build (ATKB_DEBUG_BOUNDS): an index
+ * outside its buffer sets a bit of g_atkb_debug_fault and the access is
+ * skipped; atkb_pfb_debug_fault reads and clears the word. In the normal
+ * build IDX_OK is constant true and costs nothing. */
+#ifdef ATKB_DEBUG_BOUNDS
+__device__ unsigned g_atkb_debug_fault;
+__device__ __forceinline__ bool idx_ok(bool ok) {
+    if (!ok) atomicOr(&g_atkb_debug_fault, ATKB_FAULT_INDEX);
+    return ok;
+}
+#define IDX_OK(c) idx_ok(c)
+[[maybe_unused]] inline unsigned take_debug_fault() {
+    unsigned v = 0, z = 0;
+    if (cudaMemcpyFromSymbol(&v, g_atkb_debug_fault, sizeof v) != cudaSuccess) return ATKB_FAULT_INDEX;
+    if (v) cudaMemcpyToSymbol(g_atkb_debug_fault, &z, sizeof z);
+    return v;
+}
+#else
+#define IDX_OK(c) true
+#endif
+
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {

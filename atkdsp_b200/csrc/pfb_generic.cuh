@@ -79,7 +79,8 @@ __device__ __forceinline__ void generic_pass(const double2 *__restrict__ src, do
         }
         dft_any<R>(v);
 #pragma unroll
-        for (int r = 0; r < R; ++r) d[r * Ns] = v[r];
+        for (int r = 0; r < R; ++r)
+            if (IDX_OK((j - k) * R + k + r * Ns < (unsigned)M)) d[r * Ns] = v[r];
     }
 }
 
@@ -102,7 +103,7 @@ __device__ __noinline__ void direct_pass(const double2 *__restrict__ src, double
             e += inc;
             if (e >= NsR) e -= NsR;
         }
-        dst[tt * M + (j - k) * R + k + o * Ns] = acc;
+        if (IDX_OK(e < NsR && (j - k) * R + k + o * Ns < (unsigned)M)) dst[tt * M + (j - k) * R + k + o * Ns] = acc;
     }
 }
 
@@ -124,7 +125,7 @@ __device__ __forceinline__ void generic_tile(const atkb_job &J, const atkb_bank 
             float2 x[U];
 #pragma unroll
             for (int u = 0; u < U; ++u)
-                if (k0 + u < K) {
+                if (k0 + u < K && IDX_OK(base + (k0 + u) * M < J.nsrc)) {
                     h[u] = __ldg(taps + (k0 + u) * M + q);
                     x[u] = src.at(base + (k0 + u) * M);
                 }
@@ -170,8 +171,9 @@ __device__ __forceinline__ void generic_tile(const atkb_job &J, const atkb_bank 
             const float2 c = __ldg(cal + kb);
             X = cmul_rn(X, make_double2((double)c.x, (double)c.y));
         }
-        out[(long long)kb * J.ldo + J.out_col + h0 + tt] =
-            make_float2(__double2float_rn(X.x), __double2float_rn(X.y));
+        if (IDX_OK(kb < (unsigned)M && J.out_col + h0 + tt < J.ldo))
+            out[(long long)kb * J.ldo + J.out_col + h0 + tt] =
+                make_float2(__double2float_rn(X.x), __double2float_rn(X.y));
     }
 }
 

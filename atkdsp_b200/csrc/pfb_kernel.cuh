@@ -34,27 +34,6 @@ namespace {
 
 #include "pfb_dev.cuh"
 
-/* Per-thread index checks of the debug build (ATKB_DEBUG_BOUNDS): an index
- * outside its buffer sets a bit of g_atkb_debug_fault and the access is
- * skipped; atkb_pfb_debug_fault reads and clears the word. In the normal
- * build IDX_OK is constant true and costs nothing. */
-#ifdef ATKB_DEBUG_BOUNDS
-__device__ unsigned g_atkb_debug_fault;
-__device__ __forceinline__ bool idx_ok(bool ok) {
-    if (!ok) atomicOr(&g_atkb_debug_fault, ATKB_FAULT_INDEX);
-    return ok;
-}
-#define IDX_OK(c) idx_ok(c)
-inline unsigned take_debug_fault() {
-    unsigned v = 0, z = 0;
-    if (cudaMemcpyFromSymbol(&v, g_atkb_debug_fault, sizeof v) != cudaSuccess) return ATKB_FAULT_INDEX;
-    if (v) cudaMemcpyToSymbol(g_atkb_debug_fault, &z, sizeof z);
-    return v;
-}
-#else
-#define IDX_OK(c) true
-#endif
-
 /* ---- fast path: nchan = 2^n, 16 <= nchan <= 4096 ------------------------- */
 /* Shared-memory index swizzle for the 16-byte complex doubles: the low LOGP
  * index bits are XORed with the next LOGP. The first pass stores at a stride

@@ -180,3 +180,98 @@ print("clean")
     env = dict(os.environ, ATKDSP_B200_LIB=str(dbg), PYTHONPATH=f"{root}:{root / 'tests'}")
     res = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=600)
     assert res.returncode == 0 and "clean" in res.stdout, res.stdout + res.stderr
+
+
+@pytest.mark.parametrize("M,os_,K,hops,nel", [
+    (1024, 2, 12, 80, 1),                  # one CTA per hop, the job in the launch's parameters
+    (1024, 2, 12, 400, 1), (64, 1, 16, 4000, 1), (256, 2, 12, 2000, 1), (512, 4, 8, 700, 1),
+    (2048, 8, 5, 200, 1), (4096, 2, 8, 150, 1), (4096, 8, 4, 90, 1),   # the tile kernels of one shape
+    (1024, 2, 12, 80, 2), (16, 2, 8, 3000, 2),                         # ... from a table of jobs
+    (1000, 2, 12, 60, 1), (24, 2, 8, 900, 1), (1000, 2, 12, 60, 2)])   # the generic kernels
+def test_bounds_checks_of_every_route(M, os_, K, hops, nel):
+    """The uniform window and carry checks of each kernel a handle's device
+    calls take (the test above runs one of them): the same host-side injection,
+    100 samples short of what the buffers hold. The last hop's columns stay as
+    they were, window and carry are reported, and the handle works again after
+    a reset."""
+    from atkdsp_b200 import gpu
+    lib = ak.load()
+    rng = np.random.default_rng(M + hops)
+    xs = [torch.from_numpy(W_noise(rng, hops * (M // os_))).cuda() for _ in range(nel)]
+    p = ak.Pfb(FS, M, os_, K, 80.0, nel)
+    first = gpu.process_n(p, xs, nel)
+    gpu.sync(p)
+    first = first.cpu().numpy()
+    assert lib.atkdsp_gpu_pfb_faults(p.handle) == 0 and first.shape == (nel, M, hops)
+    out = torch.full((nel * M * hops,), complex(7.0, 7.0), dtype=torch.complex64, device="cuda")
+    lib.atkdsp_gpu_inject_short_window(100)
+    gpu.process_n(p, xs, nel, out=out)
+    f = lib.atkdsp_gpu_pfb_faults(p.handle)
+    assert f == (1 | 4), f                                   # a window, and the carry; nothing else
+    o = out.view(nel, M, hops).cpu().numpy()
+    assert np.all(o[:, :, -1] == complex(7.0, 7.0))
+    assert lib.atkdsp_gpu_pfb_faults(p.handle) == 0          # cleared by the query
+    p.reset()
+    gpu.process_n(p, xs, nel, out=out)
+    gpu.sync(p)
+    assert np.array_equal(out.view(nel, M, hops).cpu().numpy(), first)
+    assert lib.atkdsp_gpu_pfb_faults(p.handle) == 0
+
+
+def test_index_checked_build_runs_the_device_routes():
+    """The index-checked library through device calls past the per-hop kernel's
+    line (every fold of the tile kernels), below it, on generic banks and in
+    one batch of all of them: no index flagged, outputs as the oracle's. In a
+    child process: it loads the other library."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+    root = Path(__file__).resolve().parent.parent
+    dbg = root / "atkdsp_b200" / "lib" / "libatkdsp_b200_debug.so"
+    if not dbg.exists():
+        pytest.skip("the index-checked library is not built (make -C atkdsp_b200 debug)")
+    code = r"""
+import numpy as np, torch, atkdsp_b200 as ak
+from atkdsp_b200 import gpu
+from oracle import oracle as O
+lib = ak.load()
+assert lib.atkdsp_gpu_debug_build() == 1
+rng = np.random.default_rng(4)
+hs, xs, refs = [], [], []
+for M, os_, K, choice in ((16, 2, 8, 2), (64, 2, 8, 1), (64, 1, 16, 5), (256, 2, 12, 2), (256, 4, 8, 1), (1024, 2, 16, 1),
+                          (1024, 1, 8, 0), (1024, 8, 4, -1), (2048, 2, 6, 1), (4096, 2, 8, -1), (4096, 8, 3, -1),
+                          (8, 2, 12, -1), (24, 2, 8, -1), (192, 2, 6, -1), (1021, 1, 3, -1), (1000, 2, 12, -1)):
+    if choice >= 0:
+        assert lib.atkdsp_gpu_tune_set(M, os_, K, choice) == 0
+    p, q = ak.Pfb(2.4e6, M, os_, K), ak.Pfb(2.4e6, M, os_, K)
+    if choice >= 0:
+        lib.atkdsp_gpu_tune_set(M, os_, K, -1)
+    r = O.oracle().Pfb(2.4e6, M, os_, K)
+    hop = M // os_
+    n = min((1 << 17) // M + 9, 2100) * hop + hop // 2 + 1
+    for n in (n, 3 * hop + 1):
+        x = ((rng.standard_normal(n) + 1j * rng.standard_normal(n)) / 2).astype(np.complex64)
+        d = torch.from_numpy(x).cuda()
+        y, want = gpu.process_n(p, [d], 1), r.process(x)
+        gpu.sync(p)
+        y = y.cpu().numpy()[0]
+        assert y.shape == want.shape and np.max(np.abs(y - want)) <= 1e-5 * np.max(np.abs(want)), (M, n)
+        assert lib.atkdsp_gpu_pfb_faults(p.handle) == 0, (M, n)
+        if n > 3 * hop + 1:
+            hs.append(q)
+            xs.append(d)
+            refs.append(want)
+batch = gpu.Batch(hs)
+outs = [torch.zeros(w.size, dtype=torch.complex64, device="cuda") for w in refs]
+torch.cuda.synchronize()
+batch.process(xs, outs)
+torch.cuda.synchronize()
+for o, w in zip(outs, refs):
+    assert np.max(np.abs(o.cpu().numpy().reshape(w.shape) - w)) <= 1e-5 * np.max(np.abs(w)), w.shape
+assert lib.atkdsp_gpu_batch_faults(batch._b) == 0
+print("clean")
+"""
+    env = dict(os.environ, ATKDSP_B200_LIB=str(dbg), PYTHONPATH=f"{root}:{root / 'tests'}")
+    res = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=600)
+    assert res.returncode == 0 and "clean" in res.stdout, res.stdout + res.stderr
