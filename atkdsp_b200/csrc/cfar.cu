@@ -302,7 +302,9 @@ int grid_for(long long work) {
 
 /* bins x (groups of fr frames), two CTAs on every SM: enough to take fr */
 static bool wide_enough(long long nbins, long long nf, int fr) {
-    return (nbins + kThreads - 1) / kThreads * (nf / fr) >= 2 * 148;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    return (nbins + kThreads - 1) / kThreads * (nf / fr) >= 2LL * atkb_sm_count(dev);
 }
 
 extern "C" int atkb_cfar_raw(const float *frames, int units, long long f0, int nf, long long nbins, double *raw,

@@ -303,10 +303,11 @@ extern "C" int atkb_pfb_hops1(const atkb_job *J, const atkb_carry *C, int m, int
 }
 
 /* hops a generic CTA takes: about 1024 points (nchan 24 43 hops, 1000 one);
- * fewer when a launch of m hops would leave SMs idle */
-static int generic_hops(int nchan, long long m) {
+ * fewer when a launch of m hops would leave less than two CTAs an SM */
+static int generic_hops(int dev, int nchan, long long m) {
+    const long long wave = 2LL * atkb_sm_count(dev);
     long long gh = 1024 / nchan;
-    if (gh > (m + 295) / 296) gh = (m + 295) / 296;
+    if (gh > (m + wave - 1) / wave) gh = (m + wave - 1) / wave;
     return gh < 1 ? 1 : (int)gh;
 }
 
@@ -324,7 +325,7 @@ static int generic_launch(const atkb_job *jobs, const atkb_carry *carries, bool 
             return ATKB_E_KERNEL;
         configured[dev].store(true, std::memory_order_release);
     }
-    const int gh = generic_hops(nchan, (long long)m * njobs), groups = (m + gh - 1) / gh;
+    const int gh = generic_hops(dev, nchan, (long long)m * njobs), groups = (m + gh - 1) / gh;
     const long long grid = (long long)njobs * groups + njobs;
     if (grid > 0x7fffffffLL) return ATKB_E_ARG;
     const size_t smem = (size_t)nchan * gh * 32;
