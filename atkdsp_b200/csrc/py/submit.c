@@ -8,6 +8,9 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <stdint.h>
+#if PY_VERSION_HEX < 0x030C0000
+#error "needs Python 3.12's headers: PyObject_VectorcallMethod is outside the limited API before"
+#endif
 
 typedef int (*submit_fn)(void *s, int id, const void *d_raw, size_t n, void *d_out, size_t cap, uint64_t tag,
                          double t_arrival);

@@ -69,3 +69,34 @@ def test_same_refusals(server, monkeypatch, bad):
     a.update(bad)
     rc, seen = _both(srv, calls, monkeypatch, **a)
     assert isinstance(rc, type) and issubclass(rc, Exception) and not seen
+
+
+@pytest.mark.parametrize("version", ["0x030B00F0", "0x030900F0", None])
+def test_module_is_left_out_where_it_does_not_build(tmp_path, version):
+    """Headers of a Python before 3.12 (declaring all the module uses), or a
+    compiler that fails: make goes on, an older module is taken away, and the
+    package's loader falls back to ctypes."""
+    import shutil
+    import subprocess
+    from pathlib import Path
+    src = Path(serve.__file__).resolve().parent
+    (tmp_path / "csrc" / "py").mkdir(parents=True)
+    (tmp_path / "lib").mkdir()
+    shutil.copy(src / "Makefile", tmp_path / "Makefile")
+    shutil.copy(src / "csrc" / "py" / "submit.c", tmp_path / "csrc" / "py" / "submit.c")
+    so = tmp_path / "lib" / "_atkdsp_submit.so"
+    so.write_bytes(b"stale")
+    import os
+    os.utime(so, (1, 1))
+    args = ["make", "-C", str(tmp_path), str(so)]
+    if version is None:
+        args.append("HCC=false")
+    else:
+        import sysconfig
+        (tmp_path / "inc").mkdir()
+        (tmp_path / "inc" / "Python.h").write_text(
+            f'#include "{sysconfig.get_paths()["include"]}/Python.h"\n#undef PY_VERSION_HEX\n#define PY_VERSION_HEX {version}\n')
+        args.append(f"PY_INC={tmp_path / 'inc'} -I{sysconfig.get_paths()['include']}")
+    r = subprocess.run(args, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    assert not so.exists()
