@@ -269,7 +269,10 @@ w12_mma_kernel(const float2 *__restrict__ out, int nel, int nchan, long long m, 
                float2 *__restrict__ R, uint32_t *__restrict__ counts, float *__restrict__ pwr,
                float *__restrict__ mean_pwr) {
     constexpr int G = 8 / NR, STEP = 4 * G, U = MMA_U;
-    __shared__ double part[MMA_WARPS][2][64];
+    /* the warps' sums, 1 KB each and no more than there are warps: the CTAs fit
+     * beside the tile kernel's of another stream */
+    extern __shared__ double part_of[];
+    double (*part)[2][64] = (double (*)[2][64])part_of;
     __shared__ double diag[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int row = lane >> 2, el = row % NR;
@@ -346,9 +349,9 @@ w12_mma_kernel(const float2 *__restrict__ out, int nel, int nchan, long long m, 
 }
 
 /* Warps per channel: the most of 16, 8 and 4 that leaves each three turns of
- * the loop (256 / NR hops a turn). A long run is bound by the loads in flight,
- * a short one by the reduction over the warps and, with many channels, by how
- * many CTAs an SM holds. us at 4 / 8 / 16 warps: 8 elements x 1024 channels x
+ * the loop (256 / NR hops a turn), two where the channels leave SMs idle. A
+ * long run is bound by the loads in flight, a short one by the reduction over
+ * the warps and, with many channels, by how many CTAs an SM holds. us at 4 / 8 / 16 warps: 8 elements x 1024 channels x
  * 20,000 hops 902 / 651 / 358 (9 to 32 elements' kernel 727), 4 x 64 x 200,000
  * 1085 / 557 / 304 (537), 8 x 4096 x 1000 102 / 83 / 95, 8 x 2048 x 256 19 /
  * 20 / 35, 2 x 4096 x 256 19 / 30 / 61. */
@@ -356,11 +359,11 @@ template <int NR>
 int w12_mma(const void *out, unsigned nel, unsigned nchan, size_t m, const uint8_t *gate, void *R,
             uint32_t *counts, float *pwr, float *mean_pwr, cudaStream_t s) {
     const int grid = (int)(nchan < 4096 ? nchan : 4096);
-    constexpr size_t turns = 3 * MMA_U * 4 * (8 / NR);
+    const size_t turns = (size_t)(nchan <= 512 ? 2 : 3) * MMA_U * 4 * (8 / NR);
     int warps = MMA_WARPS;
     while (warps > 4 && m < warps * turns) warps /= 2;
-    w12_mma_kernel<NR><<<grid, 32 * warps, 0, s>>>((const float2 *)out, (int)nel, (int)nchan, (long long)m, gate,
-                                                   (float2 *)R, counts, pwr, mean_pwr);
+    w12_mma_kernel<NR><<<grid, 32 * warps, (size_t)warps * 2 * 64 * sizeof(double), s>>>(
+        (const float2 *)out, (int)nel, (int)nchan, (long long)m, gate, (float2 *)R, counts, pwr, mean_pwr);
     return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;
 }
 

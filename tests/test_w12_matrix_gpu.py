@@ -82,8 +82,8 @@ def test_infinities_and_nan_stay_in_their_entries(nel):
     assert got[3, 1, 1].real == np.inf and np.isnan(got[5, 0, 0].real)
 
 
-@pytest.mark.parametrize("nel,ms", [(2, (3071, 3072, 6143, 6145)), (3, (1535, 1536, 3073)), (4, (3071, 3072)),
-                                    (5, (767, 1537)), (8, (767, 768, 1535, 1536, 9001))])
+@pytest.mark.parametrize("nel,ms", [(2, (2047, 2048, 4095, 4097)), (3, (1023, 1024, 2049)), (4, (2047, 2048)),
+                                    (5, (511, 1025)), (8, (511, 512, 1023, 1024, 9001))])
 def test_runs_around_the_warp_counts(nel, ms):
     """4, 8 and 16 warps a channel: hop counts around the lines between them,
     where a warp's run is shortest and the last may be empty."""
