@@ -18,8 +18,13 @@ extern "C" int atkb_get_device(int *dev) { return st(cudaGetDevice(dev)); }
 extern "C" int atkb_set_device(int dev) { return st(cudaSetDevice(dev)); }
 
 extern "C" int atkb_sm_count(int dev) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 1;
+    /* asked for at every launch; a device's count does not change */
+    static std::atomic<int> known[64];
+    const bool slot = dev >= 0 && dev < 64;
+    int n = slot ? known[dev].load(std::memory_order_relaxed) : 0;
+    if (n > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 1;
+    if (slot) known[dev].store(n, std::memory_order_relaxed);
     return n;
 }
 
