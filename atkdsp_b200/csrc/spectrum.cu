@@ -78,9 +78,14 @@ struct SpecPass {
     }
 };
 
-/* MODE 0 / 1 / 2: reduce with the max / min / average detector; 3: stats */
-template <int MODE, int LOGN>
-__global__ void __launch_bounds__(SP_NT, MODE == 3 ? 1 : 2)
+/* MODE 0 / 1 / 2: reduce with the max / min / average detector; 3: stats.
+ * PER_SM CTAs an SM: at two the 64 registers spill a little, which a launch
+ * that fills the chip with frames of 2048 or 4096 points (or 64) makes up for
+ * and others do not: us at one / two, one detector, 2^23 samples, n 4096 hop
+ * 2048 119 / 110, n 64 34 / 32, n 256 hop 128 63 / 73, n 1024 hop 512 89 / 94;
+ * a single frame of 2048 points 11.2 / 12.5. */
+template <int MODE, int LOGN, int PER_SM>
+__global__ void __launch_bounds__(SP_NT, PER_SM)
 spec_frames_kernel(const float2 *__restrict__ in, long long frames, long long hop, const float *__restrict__ win,
                    const double2 *__restrict__ tw, int per, void *__restrict__ part) {
     extern __shared__ double2 smem[];
@@ -251,18 +256,22 @@ int spec_run_n(const void *in, long long frames, long long hop, const float *win
                void *part, float *o0, float *o1, float *o2, float *o3, cudaStream_t s) {
     constexpr int n = 1 << LOGN;
     constexpr int smem = SP_NT * 8 * 16;
+    constexpr int full = MODE < 3 && (LOGN == 6 || LOGN >= 11) ? 2 : 1;
     /* the attribute is idempotent: concurrent first callers may both set it */
     static std::atomic<bool> configured[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return ATKB_E_NODEV;
     if (!configured[dev].load(std::memory_order_acquire)) {
-        if (cudaFuncSetAttribute(spec_frames_kernel<MODE, LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-            cudaSuccess)
+        if (cudaFuncSetAttribute(spec_frames_kernel<MODE, LOGN, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 smem) != cudaSuccess ||
+            cudaFuncSetAttribute(spec_frames_kernel<MODE, LOGN, full>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 smem) != cudaSuccess)
             return ATKB_E_KERNEL;
         configured[dev].store(true, std::memory_order_release);
     }
-    spec_frames_kernel<MODE, LOGN><<<nblk, SP_NT, smem, s>>>((const float2 *)in, frames, hop, win,
-                                                             (const double2 *)tw, per, part);
+    const auto frames_kernel = nblk > atkb_sm_count(dev) ? spec_frames_kernel<MODE, LOGN, full>
+                                                         : spec_frames_kernel<MODE, LOGN, 1>;
+    frames_kernel<<<nblk, SP_NT, smem, s>>>((const float2 *)in, frames, hop, win, (const double2 *)tw, per, part);
     spec_final_kernel<MODE><<<(n + SF_BINS - 1) / SF_BINS, SF_BINS * SF_SL, 0, s>>>((const double *)part, nblk, n,
                                                                                    frames, o0, o1, o2, o3);
     return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;
