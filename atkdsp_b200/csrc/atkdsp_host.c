@@ -882,7 +882,11 @@ static int run_step_up(atkdsp_pfb *p, unsigned nel, const void *const *ins, size
     {
         /* nel jobs: tile_start[nel] is their total (the kernel reads
          * tile_start[njobs]); the same launch copies the nel carries */
-        const int work = (int)nel * tiles + (int)nel;
+        /* a CTA for every tile and carry; more for the parts of a carry only
+         * where they leave an SM to each tile */
+        const int parts = (int)nel * tiles + ((int)nel << (nel <= ATKB_FEW_JOBS ? ATKB_CARRY_SPLIT : 0));
+        const int sms = atkb_sm_count(p->dev), least = (int)nel * tiles + (int)nel;
+        const int most = parts < sms ? parts : sms, work = most > least ? most : least;
         if (generic)
             rc = atkb_pfb_generic(tbl_jobs(tb), tbl_carry(tb, p->max_nel), 0, (int)nel, (int)m, (int)p->nchan,
                                   p->d_counters, stream);

@@ -199,6 +199,10 @@ int  atkb_pfb_max_smem(void);
  * counters: ATKB_NCOUNTERS ints, zero before the first launch; the kernel
  * leaves them zero again. */
 #define ATKB_NCOUNTERS 4
+/* a launch of at most this many jobs copies each carry in 2^ATKB_CARRY_SPLIT
+ * parts (many jobs have as many CTAs at it without, and each part is a claim) */
+#define ATKB_FEW_JOBS 32
+#define ATKB_CARRY_SPLIT 3
 int  atkb_pfb_launch(const atkb_job *d_jobs, const int *d_tile_start, const atkb_carry *d_carry,
                      int njobs, int *d_counters, int grid, int smem_bytes, const atkb_bank *B, void *stream);
 /* the same with the job count read from device memory (at most the given

@@ -47,11 +47,11 @@ namespace {
 /* Every shape's tile, and the generic banks', is a function of its own, so
  * that each gets the 64 registers for itself: with all of them inline one
  * allocation served 50 shapes with 1.5 to 1.9 KB of spills, and a change in
- * any one (the generic branch above all) moved the others by up to 12 %.
- * us, all inline / apart: 64 uneven streams 1090 / 1070, another 64 1271 /
- * 1233, 256 of them 5293 / 5181. The generic tile loads one tap at a time:
- * eight in flight need more registers than are left. Six scales of 8 to 256
- * channels, chunks of 65,536 samples: 1255 / 1450 MS/s. */
+ * any one (the generic branch above all) moved the others. us, all inline /
+ * apart: 64 uneven streams 1068 / 1062, another 64 1231 / 1211, 256 of them
+ * 5209 / 5169. The generic tile loads one tap at a time: eight in flight need
+ * more registers than are left (six scales of 8 to 256 channels, chunks of
+ * 65,536 samples: 1255 MS/s at eight, 1450 at one). */
 __device__ __noinline__ void tile_generic(const atkb_job &__restrict__ J, const atkb_bank &__restrict__ B,
                                           long long h0, int nvalid) {
     extern __shared__ double2 sm[];
@@ -66,6 +66,9 @@ __device__ __noinline__ void tile_of(const atkb_job &__restrict__ J, const atkb_
 }
 
 struct AllShapes {
+    static __device__ __forceinline__ void carry(const Src &src, float2 *dst, long long from, long long len) {
+        carry_runs<NT>(src, dst, from, len);
+    }
     static __device__ __forceinline__ void run(int key, const atkb_job &J, const atkb_bank &SB, long long h0,
                                                int nvalid, double2 *, float2 *) {
         switch (key) {

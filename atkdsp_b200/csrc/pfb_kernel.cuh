@@ -994,7 +994,8 @@ __device__ __forceinline__ void fetch_tile(const atkb_job *__restrict__ jobs, co
     if (lane == 0) s_local[slot] = tile - tile_start[lo];
 }
 
-/* RUN::run(key, ...) does one tile, or nothing for key -1, a tile to skip */
+/* RUN::run(key, ...) does one tile, or nothing for key -1, a tile to skip;
+ * RUN::carry copies (part of) a state carry */
 template <class RUN>
 __device__ __forceinline__ void tiles_loop(const atkb_job *__restrict__ jobs, const int *__restrict__ tile_start,
                                            const atkb_carry *__restrict__ carries, int njobs,
@@ -1051,16 +1052,20 @@ __device__ __forceinline__ void tiles_loop(const atkb_job *__restrict__ jobs, co
      * atkdsp_gpu_pfb_process_w12) may be scheduled once every CTA is here; it
      * waits for this grid's completion before it reads anything */
     asm volatile("griddepcontrol.launch_dependents;");
-    /* then the state carries, one job's per claim, the CTA's threads copying
-     * s[from, from + len) into the other state buffer (no tile reads it) */
+    /* then the state carries, an eighth of a job's per claim where the jobs are
+     * few (else a whole one), the CTA's threads copying its part of
+     * s[from, from + len) into the other state buffer (no tile reads it). One
+     * CTA for a whole carry set the time of short launches with long prototypes:
+     * nchan 2048, 1x, 40 taps, 262,147 samples 42.7 us, so 27.7. */
+    const int sh = njobs <= ATKB_FEW_JOBS ? ATKB_CARRY_SPLIT : 0;
     __shared__ int s_carry;
     for (;;) {
         if (threadIdx.x == 0) s_carry = atomicAdd(&counters[2], 1);
         __syncthreads();
         const int ci = s_carry;
         __syncthreads();                  /* read before thread 0 claims again */
-        if (ci >= njobs) break;
-        const atkb_carry &C = carries[ci];
+        if (ci >> sh >= njobs) break;
+        const atkb_carry &C = carries[ci >> sh];
         const Src src{(const float2 *)C.state, C.in, C.head, C.in_kind, C.cre, C.cim, C.kscale};
         float2 *dst = (float2 *)C.dst;
         const long long from = C.from, len = C.len;
@@ -1068,7 +1073,8 @@ __device__ __forceinline__ void tiles_loop(const atkb_job *__restrict__ jobs, co
             if (threadIdx.x == 0) atomicOr((unsigned *)&counters[ATKB_FAULT_WORD], ATKB_FAULT_CARRY);
             continue;
         }
-        carry_copy<NT>(src, dst, from, len);
+        const long long part = (len + (1 << sh) - 1) >> sh, at = part * (ci & ((1 << sh) - 1));
+        if (at < len) RUN::carry(src, dst + at, from + at, min(part, len - at));
     }
     if (threadIdx.x == 0) {
         __threadfence();

@@ -17,6 +17,9 @@ namespace {
 
 template <int KEY>
 struct OneShape {
+    static __device__ __forceinline__ void carry(const Src &src, float2 *dst, long long from, long long len) {
+        carry_copy<NT>(src, dst, from, len);
+    }
     static __device__ __forceinline__ void run(int key, const atkb_job &J, const atkb_bank &SB, long long h0,
                                                int nvalid, double2 *sm, float2 *to) {
         if (key == KEY) run_tile<KEY>(J, SB, h0, nvalid, sm, to);
