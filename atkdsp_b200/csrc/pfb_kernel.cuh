@@ -385,16 +385,15 @@ struct PairStaged {                    /* the padded shared-memory window */
     }
 };
 
-/* Taps a turn of the paired fold's loop; 0 leaves it to the compiler, which in
- * the kernels of one shape (pfb_one.cu) chose worse for a few than it had in
- * the kernel of every shape: us there / left to it / as here, 3,000,001
- * samples, nchan 4096 4x 12 taps 187 / 192 / 178, 4096 4x 16 199 / 205 / 193,
- * 2048 1x 16 50.7 / 53.6 / 51.7, 16 4x 16 142 / 148 / 137, 16 2x 5 66 / 71 / 64.
- * nchan 4096 1x is best at four (10,000,001 samples, 12 taps: 165 / 167 / 165,
- * one tap 167). */
+/* Taps a turn of the paired fold's loop in the kernels of one shape
+ * (pfb_one.cu); 0 leaves it to the compiler, as in the kernel of every shape.
+ * us left to it / as here, 3,000,001 samples: nchan 4096 4x 12 taps 189 / 177,
+ * 4x 16 199 / 189, 2x 16 97.4 / 94.6; 2048 1x 12 taps 45.4 / 43.3; nchan 16 4x 5
+ * taps 115 / 110, 4x 16 137 / 134. The other shapes' loops are as good as any. */
 __host__ __device__ constexpr int fold_unroll(int logm, int logos) {
 #ifdef ONE_LOGM
-    return logm == 4 ? 2 : logm == 12 ? (logos == 0 ? 4 : 1) : logm == 11 && logos == 0 ? 1 : 0;
+    if (logm == 4) return logos > 0 ? 2 : 0;
+    return (logm == 12 && logos > 0) || (logm == 11 && logos == 0) ? 1 : 0;
 #else
     return 0;
 #endif
