@@ -611,7 +611,9 @@ atkdsp_pfb *atkb_pfb_create_internal(double fs, unsigned nchan, unsigned oversam
     if (rc == ATKB_OK) rc = atkb_memset(p->d_counters, 0, ATKB_NCOUNTERS * sizeof(int), p->stream);
     if (rc == ATKB_OK) rc = atkb_stream_sync(p->stream);
     if (rc != ATKB_OK) { atkdsp_pfb_destroy(p); return NULL; }
-    p->grid = atkb_pfb_grid(p->dev, p->bank.smem_bytes, &p->bank);
+    /* a generic bank's handle launches no tile kernel: loading it here took
+     * longer than the handle's first call */
+    p->grid = p->bank.plan.fast || p->bank.plan.big ? atkb_pfb_grid(p->dev, p->bank.smem_bytes, &p->bank) : 1;
     if (p->grid < 1) { atkdsp_pfb_destroy(p); return NULL; }
     p->lc = 0;
     p->b = 0;
