@@ -17,7 +17,7 @@ struct atkdsp_gpu_spectrum {
     int logn;
     int maxblk;                   /* partial lines held */
     void *d_tw;                   /* n double2: (cos, -sin)(2 pi j / n) */
-    void *d_part;                 /* maxblk * 4 * n doubles */
+    void *d_part;                 /* maxblk lines of n doubles, or half as many of four planes */
 };
 
 ATKDSP_API void atkdsp_gpu_spectrum_destroy(atkdsp_gpu_spectrum *p) {
@@ -38,7 +38,7 @@ ATKDSP_API atkdsp_gpu_spectrum *atkdsp_gpu_spectrum_create(size_t n) {
     double *tw = (double *)malloc(2 * n * sizeof(double));
     if (!tw) rc = ATKB_E_NOMEM;
     if (rc == ATKB_OK) rc = atkb_malloc(&p->d_tw, 2 * n * sizeof(double));
-    if (rc == ATKB_OK) rc = atkb_malloc(&p->d_part, (size_t)p->maxblk * 4 * n * sizeof(double));
+    if (rc == ATKB_OK) rc = atkb_malloc(&p->d_part, (size_t)p->maxblk * 2 * n * sizeof(double));
     if (rc == ATKB_OK) {
         size_t j;
         for (j = 0; j < n; ++j) {
