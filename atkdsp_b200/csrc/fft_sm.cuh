@@ -110,14 +110,6 @@ __device__ void fft_b(double2 *sm, int logn, int nb, const double2 *__restrict__
     }
 }
 
-/* bin k of a channel's decimating fold of one spectrum (float, j ascending,
- * the reference's rounded expression, src/channelizer.c:707-716). The bins
- * k + j*M + shift run up to nfft and then wrap once: two runs, each a
- * fixed stride (M is a template parameter, so the unrolled loads carry it
- * as an immediate offset). SM: the spectrum is the fused kernel's shared
- * one, bin b of this block at shared address xs + b * 8 * OSX_G; else
- * global, bin b at X[b]. */
-
 /* ---- radix-8 transforms in a swizzled layout --------------------------------
  * Element p of a transform lives at sm[swz(p)]: the low 3 index bits XORed
  * with the next 3, so the stride-8 stores of a radix-8 pass and the

@@ -58,12 +58,11 @@ __device__ __forceinline__ float2 lds8(unsigned a) {
  * k + j*M + shift, which run up to nfft (a power of two) and wrap once.
  * The fused kernel's spectrum, bin b of this block at shared address
  * xs + b * 8 * OSX_G. The filter does not wrap, so its values come in batches
- * a batch ahead: with the batch's own loads only, a batch waited for L2 (the
- * channels' filters are larger than the L1 that the spectra leave): 90 to 108
- * cycles a term a warp with 16 warps, now 80 to 85, where the shared and L1
- * load path is the bound. 64 channels of nfft 4096, 512 blocks: the group
- * kernel cold 235 -> 180 us (four of a batch in flight are slower than eight,
- * sixteen spill). */
+ * a batch ahead (the channels' filters are larger than the L1 that the spectra
+ * leave, and a batch would wait for L2); the shared and L1 load path bounds it.
+ * 64 channels of nfft 4096, 512 blocks: the group kernel cold 235 us without
+ * the batch ahead, 180 with (four in flight are slower than eight, sixteen
+ * spill). */
 template <int LOGM>
 __device__ __forceinline__ double2 fold_shared(unsigned xs, const float2 *__restrict__ H, int k, int decim, int shift,
                                                int nfft) {

@@ -2,10 +2,8 @@
  * through fold, mixed-radix Stockham passes between two buffers, epilogue.
  * Include after pfb_dev.cuh inside a namespace.
  *
- * Radices 2, 3, 4, 5, 7 and 8 are butterflies in registers; any other
- * prime factor is a direct DFT. (With the radix a run-time number the
- * butterfly's values lived in local memory, and radix 5 was a direct DFT with
- * a 64-bit remainder per term: nchan 1000 = 8 * 5^3 ran at 5.3 GS/s.) */
+ * Radices 2, 3, 4, 5, 7 and 8 are butterflies in registers (the radix a
+ * template argument); any other prime factor is a direct DFT. */
 #ifndef ATKB_PFB_GENERIC_CUH
 #define ATKB_PFB_GENERIC_CUH
 

@@ -1,12 +1,11 @@
 /* The tile kernel for launches whose tiles are all of one shape (a handle's
- * call, an array's, the fused front end): registers for that shape alone. In
- * the kernel of every shape at 64 registers a thread one shape's needs spill
- * another's (1.5 KB of spills against 20-140 bytes in these). Compiled once
+ * call, an array's, the fused front end): registers for that shape alone (4 to
+ * 152 bytes of spills). Compiled once
  * per nchan, 2^ONE_LOGM, by the Makefile (an object each, built side by side);
  * without ONE_LOGM it is the table of them.
  *
- * One stream of 2^23 samples, nchan 1024, 2x, 16 taps: 204.5 -> 197.7 us; eight
- * elements at nchan 2048 with W1/W2: 202 -> 194 us. */
+ * One stream of 8,388,301 samples, nchan 1024, 2x, 16 taps: 204.5 us through the
+ * kernel of every shape, 196.4 here; eight elements at nchan 2048: 141, 134. */
 #ifdef ONE_LOGM
 #include "pfb_kernel.cuh"
 
