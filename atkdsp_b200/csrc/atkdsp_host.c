@@ -838,7 +838,7 @@ static int run_step_up(atkdsp_pfb *p, unsigned nel, const void *const *ins, size
      * the job in the launch's parameters */
     const int generic = !p->bank.plan.fast && !big;
     if (nel == 1 && !up_extra &&
-        (generic || (!J[0].w2 && m <= atkb_hops1_max((unsigned)p->bank.K) && m * p->nchan <= ATKB_HOPS1_POINTS &&
+        (generic || (!J[0].w2 && m <= atkb_hops1_max((unsigned)p->bank.K, (unsigned)p->bank.os) && m * p->nchan <= ATKB_HOPS1_POINTS &&
                      atkb_pfb_hops_ok(&p->bank)))) {
         rc = generic ? atkb_pfb_generic(&J[0], &C[0], 1, 1, (int)m, (int)p->nchan, p->d_counters, stream)
                      : atkb_pfb_hops1(&J[0], &C[0], (int)m, (int)p->nchan, p->d_counters, stream);

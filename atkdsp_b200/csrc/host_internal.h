@@ -33,8 +33,12 @@ atkdsp_pfb *atkb_pfb_create_served(double fs, unsigned nchan, unsigned oversampl
  * long prototypes, whose taps and samples each hop reads for itself. 2048 hops:
  * nchan 64, 2x, 16 taps 15.5 / 12.4, nchan 32, 1x, 20 taps 14.8 / 14.5, 32 taps
  * 16.6 / 18.5, 128 taps 44 / 44 (2x: 30 / 43); 1536 hops: 32 taps faster at
- * nchan 16 to 64; 1024 hops: nchan 16, 1x, 128 taps 29 / 24, nchan 128 44 / 43. */
-static inline size_t atkb_hops1_max(unsigned taps) { return taps <= 20 ? 2048 : taps <= 32 ? 1536 : 1024; }
+ * nchan 16 to 64; 1024 hops: nchan 16, 1x, 128 taps 29 / 24, nchan 128 44 / 43.
+ * Beyond 4x no fold of the tile kernel shares samples between hops: nchan 32,
+ * 8x, 2048 hops, 128 taps 219 / 38. */
+static inline size_t atkb_hops1_max(unsigned taps, unsigned os) {
+    return taps <= 20 || os > 4 ? 2048 : taps <= 32 ? 1536 : 1024;
+}
 /* ... and write at most this many outputs straight into pinned host memory */
 #define ATKB_DIRECT_OUT 2048
 

@@ -46,7 +46,8 @@ def test_device_calls_equal_the_tile_kernel(M, os_, K, fmt):
         assert ak.load().atkdsp_gpu_pfb_faults(a.handle) == 0
 
 
-@pytest.mark.parametrize("M,os_,K,line", [(16, 2, 21, 1536), (32, 1, 32, 1536), (32, 2, 33, 1024), (16, 1, 40, 1024)])
+@pytest.mark.parametrize("M,os_,K,line", [(16, 2, 21, 1536), (32, 1, 32, 1536), (32, 2, 33, 1024), (16, 1, 40, 1024),
+                                          (64, 8, 40, 2048)])
 def test_long_prototypes_around_their_line(M, os_, K, line):
     """More taps a branch move the line to fewer hops; on both sides of it the
     outputs and the carried state are the tile kernel's."""
