@@ -255,7 +255,6 @@ __global__ void cov_reset_kernel(float2 *R, uint32_t *counts, int nel, int nchan
  * first figure) and the samples' trip from L2. us, the tile-per-thread kernel
  * and this one: 8 elements x 2048 channels x 513 hops 88.3, 30.2; 8 x 256 x
  * 4097 53.5, 26.9; 4 x 2048 x 513 76.1, 20.2; 2 x 1024 x 2000 23.9, 15.6. */
-#define MMA_WARPS 16
 #define MMA_U 8          /* loads in flight a lane */
 __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
@@ -263,18 +262,18 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
                  : "d"(a), "d"(b));
 }
 
-template <int NR>
-__global__ void __launch_bounds__(32 * MMA_WARPS)
+template <int NR, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS)
 w12_mma_kernel(const float2 *__restrict__ out, int nel, int nchan, long long m, const uint8_t *__restrict__ gate,
                float2 *__restrict__ R, uint32_t *__restrict__ counts, float *__restrict__ pwr,
                float *__restrict__ mean_pwr) {
     constexpr int G = 8 / NR, STEP = 4 * G, U = MMA_U;
-    /* the warps' sums, 1 KB each and no more than there are warps: the CTAs fit
-     * beside the tile kernel's of another stream */
-    extern __shared__ double part_of[];
-    double (*part)[2][64] = (double (*)[2][64])part_of;
+    /* 1 KB a warp and no more than there are warps: the CTAs fit beside the tile
+     * kernel's of another stream. (Given at the launch instead, it ran 8 elements
+     * x 16 channels x 20,000 hops in 141 us for 66.) */
+    __shared__ double part[WARPS][2][64];
     __shared__ double diag[8];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = WARPS;
     const int row = lane >> 2, el = row % NR;
     const long long at = (row / NR) * 4 + (lane & 3);        /* the lane's hop of a step */
     /* each warp's run: an equal share of the steps */
@@ -348,7 +347,7 @@ w12_mma_kernel(const float2 *__restrict__ out, int nel, int nchan, long long m, 
     }
 }
 
-/* Warps per channel: the most of 16, 8 and 4 that leaves each three turns of
+/* Warps per channel: the most of 16, 8 and 4 that leaves each six turns of
  * the loop (256 / NR hops a turn), two where the channels leave SMs idle. A
  * long run is bound by the loads in flight, a short one by the reduction over
  * the warps and, with many channels, by how many CTAs an SM holds. us at 4 / 8 / 16 warps: 8 elements x 1024 channels x
@@ -359,11 +358,14 @@ template <int NR>
 int w12_mma(const void *out, unsigned nel, unsigned nchan, size_t m, const uint8_t *gate, void *R,
             uint32_t *counts, float *pwr, float *mean_pwr, cudaStream_t s) {
     const int grid = (int)(nchan < 4096 ? nchan : 4096);
-    const size_t turns = (size_t)(nchan <= 512 ? 2 : 3) * MMA_U * 4 * (8 / NR);
-    int warps = MMA_WARPS;
-    while (warps > 4 && m < warps * turns) warps /= 2;
-    w12_mma_kernel<NR><<<grid, 32 * warps, (size_t)warps * 2 * 64 * sizeof(double), s>>>(
-        (const float2 *)out, (int)nel, (int)nchan, (long long)m, gate, (float2 *)R, counts, pwr, mean_pwr);
+    const size_t turns = (size_t)(nchan <= 512 ? 2 : 6) * MMA_U * 4 * (8 / NR);
+#define MMA(WARPS)                                                                                            \
+    w12_mma_kernel<NR, WARPS><<<grid, 32 * WARPS, 0, s>>>((const float2 *)out, (int)nel, (int)nchan,          \
+                                                          (long long)m, gate, (float2 *)R, counts, pwr, mean_pwr)
+    if (m >= 16 * turns) MMA(16);
+    else if (m >= 8 * turns) MMA(8);
+    else MMA(4);
+#undef MMA
     return cudaGetLastError() == cudaSuccess ? ATKB_OK : ATKB_E_KERNEL;
 }
 
